@@ -621,13 +621,11 @@ def bench_strategies(torch, ops, dev, xs, w, capture, timed, med, event_us, peak
         _progress(f"  grouped FFN {n_exp} experts timed")
         variants = None
         if n_exp == 8:
-            # the same shape on the one-CTA kernel (two-tile units), same box, same protocol
+            # the same shape with one MMA-issuing thread, same box, same protocol
             from moe_routers_b200._lib import lib as _l
             mode = _l.moe_set_gemm_mode(-1)
-            _l.moe_set_gemm_mode(mode & ~1)
-            variants = {"one_cta_kernel_us": ffn_graph_us()}
             _l.moe_set_gemm_mode(mode & ~2)
-            variants["two_cta_one_issuer_us"] = ffn_graph_us()
+            variants = {"one_issuer_us": ffn_graph_us()}
             _l.moe_set_gemm_mode(mode)
             # context only: the library batched GEMM on the same operands, same protocol, without the
             # activation (what the peak in MEASURED_PEAKS.json was measured with)

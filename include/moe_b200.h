@@ -15,13 +15,10 @@
  *     with different workspaces are independent (moe_pack_static, which owns
  *     its scratch, says what it shares);
  *   - environment switches, read once per process, all default to the fast
- *     path: MOE_B200_PDL=0 (no programmatic dependent launch between the
- *     route kernels; moe_set_pdl changes it at run time); grouped GEMM
- *     variants, also changed at run time by moe_set_gemm_mode: MOE_B200_CTA2=0
- *     (no two-CTA kernel), MOE_B200_CTA2_ISSUERS=1 (one MMA-issuing thread
- *     in it), MOE_B200_PAIR=0 (single-tile work units), MOE_B200_M64=0
- *     (128-row tiles only), MOE_B200_GEMM_PRODUCERS=1 (one TMA-issuing
- *     warp); MOE_B200_ROUTER_BULK=0 (router kernel: split-K partials exchanged
+ *     path: MOE_B200_PDL=0 (no programmatic dependent launch; moe_set_pdl
+ *     changes it at run time); MOE_B200_CTA2_ISSUERS=1 (one MMA-issuing
+ *     thread in the grouped GEMM, also moe_set_gemm_mode);
+ *     MOE_B200_ROUTER_BULK=0 (router kernel: split-K partials exchanged
  *     with remote stores also where a bulk copy would do),
  *     MOE_B200_ROUTER_PREFETCH=0 (no L2 prefetch of the tokens ahead of the
  *     dependency wait);
@@ -83,8 +80,8 @@ int moe_set_wait_limit(void* workspace, size_t workspace_bytes, unsigned long lo
  * count when they are captured).  Measurement helper; no counterpart in the reference. */
 long long moe_launch_count(void);
 
-/* Programmatic dependent launch between the kernels of a route (the scatter may start its input
- * prefetch under the router kernel's epilogue): 0 = plain stream order, non-zero = on (default,
+/* Programmatic dependent launch between the kernels of the library (the scatter may start its input
+ * prefetch under the router kernel's epilogue, a GEMM sets itself up under the kernel before it): 0 = plain stream order, non-zero = on (default,
  * unless MOE_B200_PDL=0 is in the environment).  Process-wide; takes effect for launches issued
  * after the call.  Measurement helper; no counterpart in the reference. */
 int moe_set_pdl(int enabled);
@@ -94,11 +91,11 @@ int moe_set_pdl(int enabled);
  * after the call (process-wide) and returns the previous one; a negative mode only reads it.
  * Measurement and test helper; no counterpart in the reference. */
 enum {
-  MOE_GEMM_TWO_CTA = 1,       /* two-CTA kernel (tcgen05 cta_group::2) for experts with >= 512 rows on average */
-  MOE_GEMM_TWO_ISSUERS = 2,   /* two MMA-issuing threads in the two-CTA kernel */
-  MOE_GEMM_TILE_PAIRS = 4,    /* one-CTA kernel: two 128-row tiles per work unit for such experts */
-  MOE_GEMM_M64 = 8,           /* one-CTA kernel: a last tile of <= 64 rows as UMMA M=64 */
-  MOE_GEMM_TWO_PRODUCERS = 16,/* one-CTA kernel: second TMA-issuing warp for single-tile units */
+  MOE_GEMM_TWO_CTA = 1,       /* no effect: every call runs on the two-CTA kernel (tcgen05 cta_group::2) */
+  MOE_GEMM_TWO_ISSUERS = 2,   /* two MMA-issuing threads */
+  MOE_GEMM_TILE_PAIRS = 4,    /* no effect (a variant of a former one-CTA kernel), as the two below */
+  MOE_GEMM_M64 = 8,
+  MOE_GEMM_TWO_PRODUCERS = 16,
   MOE_GEMM_ALL = 31
 };
 int moe_set_gemm_mode(int mode);
@@ -283,7 +280,7 @@ int moe_grouped_gemm(const void* a, const void* w, void* c, const int32_t* offse
  * dense C.  The addresses may point into another GPU's memory mapped into this process
  * (moe_ipc_open): the expert-parallel layer passes the table built by moe_ep_row_targets so that the
  * second expert GEMM returns every result row to the packed slot of the rank it came from, from
- * inside the GEMM kernel (128-byte row pieces, plain stores).
+ * inside the GEMM kernel (256-byte row pieces, plain stores).
  * Replaces, together with moe_ep_row_targets: the per-expert MLP loop followed by a separate return
  * exchange, which the reference leaves out (bench_2gpu_pcie.py:123-171, :20-25).  All other
  * arguments as moe_grouped_gemm.

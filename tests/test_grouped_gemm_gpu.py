@@ -306,3 +306,45 @@ def test_grouped_gemm_sm_margin_same_result(ops):
         torch.cuda.synchronize()
         assert ops.read_status() == 0
         assert torch.equal(got.view(torch.int16), ref.view(torch.int16)), margin
+
+
+@pytest.mark.parametrize("counts,K,N,layout,act,dtype", [
+    ([1], 8, 16, "nk", None, torch.float16),                            # the smallest call
+    ([31, 32, 33, 0, 255, 256, 257], 136, 272, "nk", "gelu", torch.float16),   # unit edges; a feature tile of 16
+    ([63, 64, 65, 127, 128, 129], 64, 464, "nk", None, torch.bfloat16),        # every token-box height; 208 features
+    ([513, 1, 1793], 128, 240, "nk", None, torch.float16),              # evenly dealt units, fewer features than a tile
+    ([17, 0, 300, 2], 200, 144, "nk", "swiglu", torch.float16),         # gate and up rows end inside a tile
+    ([90, 160, 161], 192, 320, "kn", "swiglu", torch.bfloat16),
+    ([5, 250], 72, 192, "kn", None, torch.float16),
+    ([3] * 200, 64, 64, "nk", "silu", torch.float16),                   # more experts than CTA pairs
+])
+@pytest.mark.parametrize("scattered", [False, True])
+def test_grouped_gemm_feature_major_edges(ops, counts, K, N, layout, act, dtype, scattered):
+    """Tiles of 256 features x up to 256 tokens: sizes around every edge of the unit split (32-token steps,
+    256 tokens, token boxes of 16/32/64/128 rows), feature counts that fill no tile, K tails, dense and
+    scattered rows.  Bound: the result is rounded once to the storage type (2^-11 / 2^-8 of the value) after
+    fp32 accumulation of K <= 200 products; the activations are smooth with slope <= 1.13 (times the gate's
+    or up's magnitude, inside `scale`)."""
+    off = _segments(counts)
+    rows, e = int(off[-1]), len(counts)
+    g = torch.Generator().manual_seed(rows + K + N)
+    a = torch.randn(rows, K, generator=g).to(dtype)
+    n_w = 2 * N if act == "swiglu" else N
+    w = (torch.randn(*((e, n_w, K) if layout == "nk" else (e, K, n_w)), generator=g) / K ** 0.5).to(dtype)
+    off_t = torch.from_numpy(off).cuda()
+    buf = torch.full((rows + 2, N), 7.0, dtype=dtype, device="cuda")
+    if scattered:
+        perm = torch.randperm(rows, generator=g)
+        table = (buf.data_ptr() + (perm + 1) * (N * 2)).cuda()
+        ops.grouped_gemm(a.cuda(), w.cuda(), off_t, layout=layout, activation=act, out_rows=table)
+        got = buf[1:-1].float().cpu()[perm]
+    else:
+        ops.grouped_gemm(a.cuda(), w.cuda(), off_t, layout=layout, activation=act, out=buf[1:-1])
+        got = buf[1:-1].float().cpu()
+    torch.cuda.synchronize()
+    assert ops.read_status() == 0
+    assert (buf[0] == 7.0).all() and (buf[-1] == 7.0).all()  # nothing outside the result rows
+    ref = torch.from_numpy(_ref(a, w, off, layout, act))
+    eps = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    scale = float(ref.abs().max())
+    assert ((got - ref).abs() <= 1.5 * eps * ref.abs() + 2e-5 * scale).all()
