@@ -157,27 +157,33 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
 }
-// The CTA-pair forms (`cta_group::2`, issued by one thread of the pair's even CTA): D is 256 x N, rows
+// The CTA-pair forms (`cta_group::2`, issued by the one thread of a warp of the pair's even CTA that has
+// `issue` set): D is 256 x N, rows
 // 0..127 accumulate in this CTA's TMEM and rows 128..255 in the other CTA's at the same TMEM address;
 // each CTA's shared memory holds its own 128 rows of A and its own N/2 columns of B at the same
 // offsets, which is what the descriptors (built from this CTA's addresses) name.
 __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
+                                              uint32_t accumulate, uint32_t issue) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, q;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
-// Arrive on the mbarrier at this shared-memory offset in every CTA of `cta_mask` once the pair's
-// previously issued MMAs have completed (a barrier signal, not a data copy).
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t cta_mask) {
+// Arrive on the mbarrier at this shared-memory offset in every CTA of `cta_mask` once the pair's MMAs
+// that this thread has issued have completed (a barrier signal, not a data copy).
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t cta_mask, uint32_t issue) {
   asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"(cta_mask)
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %2, 0;\n"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+      "}\n" ::"r"(bar),
+      "h"(cta_mask), "r"(issue)
       : "memory");
 }
 // 32 lanes x 16 consecutive fp32 columns: thread i of the warp gets lane
