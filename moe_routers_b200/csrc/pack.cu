@@ -169,7 +169,7 @@ pack_scatter_bulk_kernel(const char* __restrict__ x, const int32_t* __restrict__
                          int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
                          char* __restrict__ packed, int32_t* __restrict__ row_route,
                          int32_t* __restrict__ route_row, int tokens, size_t row_bytes, int experts,
-                         int top_k, int num_tiles, int nbuf, int chunk_bytes, int32_t* status,
+                         int top_k, int num_tiles, int nbuf, int chunk_bytes, int early_rows, int32_t* status,
                          char* const* __restrict__ seg_base) {
   extern __shared__ __align__(128) uint8_t s_raw[];
   uint8_t* s_buf = s_raw;                                                        // [nbuf][chunk_bytes]
@@ -208,6 +208,9 @@ pack_scatter_bulk_kernel(const char* __restrict__ x, const int32_t* __restrict__
     bytes = (uint32_t)min((size_t)chunk_bytes, row_bytes - ofs);
     return x + (size_t)(t0 + row) * row_bytes + ofs;
   };
+  // The rows may be read ahead of the dependency wait only where the caller knows that no kernel still
+  // running can be writing them.
+  if (!early_rows) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (lane == 0) {
     for (int m = 0; m < depth; ++m) {
       const int it = warp + m * kBulkIssuers;
@@ -282,11 +285,13 @@ int pick_split(int num_tiles) {
 
 }  // namespace
 
-// Shared by moe_pack and moe_route_fused: offsets + scatter from ready tile histograms.
+// Shared by moe_pack and moe_route_fused: offsets + scatter from ready tile histograms.  `early_rows`: the
+// kernel in front of the scatter neither writes `x` nor lets the scatter start before everything in front
+// of itself has completed, so the rows may be fetched under it.
 int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int tokens, int d,
                         int experts, int top_k, int32_t* counts, int32_t* offsets, void* packed,
                         int32_t* row_route, int32_t* route_row, const Workspace& ws,
-                        cudaStream_t s, void* const* seg_base = nullptr) {
+                        cudaStream_t s, void* const* seg_base = nullptr, bool early_rows = true) {
   if (tokens == 0) {
     pack_zero_kernel<<<(experts + 256) / 256, 256, 0, s>>>(counts, offsets, experts);
     return check_launch("pack_zero_kernel");
@@ -337,7 +342,8 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
       cfg.gridDim = dim3(nt, 1, 1);
       cfg.dynamicSmemBytes = smem;
       err = cudaLaunchKernelEx(&cfg, pack_scatter_bulk_kernel, xs, idx, th, tile_base, counts, offsets, ps,
-                               row_route, route_row, tokens, row_bytes, experts, top_k, nt, nbuf, chunk, st, sb);
+                               row_route, route_row, tokens, row_bytes, experts, top_k, nt, nbuf, chunk,
+                               early_rows ? 1 : 0, st, sb);
       if (err != cudaSuccess) return fail(MOE_ERR_LAUNCH, "pack_scatter_bulk_kernel: %s", cudaGetErrorString(err));
       note_launch();
       return MOE_OK;
@@ -523,7 +529,7 @@ extern "C" int moe_pack_scatter(const void* x, int elem_bytes, const int32_t* id
                 workspace_bytes_for(tokens, experts, top_k));
   Workspace ws = carve(workspace, tokens, experts);
   return launch_scan_scatter(x, elem_bytes, idx, tokens, d, experts, top_k, counts, offsets, packed, row_route,
-                             route_row, ws, static_cast<cudaStream_t>(stream), nullptr);
+                             route_row, ws, static_cast<cudaStream_t>(stream), nullptr, /*early_rows=*/false);
 }
 
 // The scatter with one destination segment per expert: the rows routed to expert e are stored, in
@@ -546,5 +552,5 @@ extern "C" int moe_pack_scatter_to(const void* x, int elem_bytes, const int32_t*
                 workspace_bytes_for(tokens, experts, top_k));
   Workspace ws = carve(workspace, tokens, experts);
   return launch_scan_scatter(x, elem_bytes, idx, tokens, d, experts, top_k, counts, offsets, nullptr, row_route,
-                             route_row, ws, static_cast<cudaStream_t>(stream), seg_base);
+                             route_row, ws, static_cast<cudaStream_t>(stream), seg_base, /*early_rows=*/false);
 }

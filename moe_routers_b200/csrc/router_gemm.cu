@@ -346,11 +346,6 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
   // Remote shared-memory traffic below needs every CTA of the cluster to be running with its
   // barriers initialised: arrive now, wait just before the first remote access.
   cluster_arrive_relaxed();
-  // Let a dependent kernel (launched with programmatic stream serialisation) start its own input
-  // prefetch as soon as it finds room; it still waits for this grid to finish before reading what
-  // we write.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-
   if (warp < kProducers) {
     // ------------------------------ TMA producers ------------------------------
     // Producer warp j owns the pipeline stages s with s % producers == j and fills them in order,
@@ -359,6 +354,11 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
     // With programmatic dependent launch this grid may start while its predecessor in the stream is
     // still running: everything above overlaps it; global memory is first touched after this wait.
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    // Let a dependent kernel (launched with programmatic stream serialisation) start its own input
+    // prefetch as soon as it finds room; it still waits for this grid to finish before reading what
+    // we write.  Only now: the scatter behind this kernel copies token rows before its own wait, and
+    // the tokens may be the output of the kernel that this one has just waited for.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (lane == 0 && warp < producers) {
       // stage, its owner and the parity of its use advance without divisions: this thread is on the
       // critical path of its fills
@@ -618,7 +618,8 @@ int check_router_args(const char* who, const void* x, const void* w, int tokens,
 
 int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int tokens, int d, int experts,
                         int top_k, int32_t* counts, int32_t* offsets, void* packed, int32_t* row_route,
-                        int32_t* route_row, const Workspace& ws, cudaStream_t s, void* const* seg_base = nullptr);
+                        int32_t* route_row, const Workspace& ws, cudaStream_t s, void* const* seg_base = nullptr,
+                        bool early_rows = true);
 
 }  // namespace moe
 

@@ -136,3 +136,25 @@ def test_pack_scatter_reuses_the_histograms_of_the_route(ops):
     side.synchronize()
     for key in ("packed", "counts", "offsets"):
         assert torch.equal(other[key], o[key]), key
+
+
+@pytest.mark.parametrize("t", [96, 1000, 4096])
+def test_route_reads_tokens_that_the_kernel_before_it_writes(ops, t):
+    """Back to back: a grouped GEMM writes the tokens (it lets dependents start early) and the route packs
+    them.  No row may be fetched before the GEMM has completed."""
+    d, k = 512, 2
+    g = torch.Generator().manual_seed(t)
+    a = torch.randn(t, 2048, generator=g).half().cuda()
+    w1 = (torch.randn(1, d, 2048, generator=g) / 45).half().cuda()
+    wr = (torch.randn(16, d, generator=g) / 22).half().cuda()
+    off = torch.tensor([0, t], dtype=torch.int32, device="cuda")
+    x = torch.empty(t, d, dtype=torch.float16, device="cuda")
+    for _ in range(5):
+        x.fill_(7.0)
+        ops.grouped_gemm(a, w1, off, layout="nk", out=x)
+        o = ops.route_fused(x, wr, k)
+        assert torch.equal(o["packed"], x[(o["row_route"] // k).long()])
+        x.fill_(7.0)
+        ops.grouped_gemm(a, w1, off, layout="nk", out=x)
+        ops.pack_scatter(x, 16, o)
+        assert torch.equal(o["packed"], x[(o["row_route"] // k).long()])
