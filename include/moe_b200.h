@@ -239,13 +239,20 @@ int moe_router_gemm_select(const void* x, const void* w_router, int dtype, int t
  *   gates = vals / (sum(vals) + eps).
  *   idx [tokens, top_k] int32, gates [tokens, top_k] float32.
  * Limits: top_k <= 8, experts <= 1024, tokens * experts * 4 bytes / (number of SMs) must fit in
- * shared memory (about 7 M matrix entries on a B200).  The kernel runs as a cooperative grid
+ * shared memory (about 7 M matrix entries on a B200).  Up to 524288 entries (experts <= 256, rounded up to
+ * 8 * 2^n) stay in the registers of one thread-block cluster; larger ones run as a cooperative grid
  * with one grid barrier per iteration; if a barrier wait gives up, the status block records it
  * and the workspace must be re-initialised with moe_workspace_init.
  */
 int moe_sinkhorn(const void* logits, int logits_dtype, int tokens, int experts, int top_k, int iters,
                  float epsilon, float temperature, int32_t* idx, float* gates, void* workspace,
                  size_t workspace_bytes, void* stream);
+
+/* The same with the result types of SinkhornRouter.forward (models/decoder_moe.py:119-123): idx int64,
+ * weights in the logits' own type (rounded once from fp32). */
+int moe_sinkhorn_router(const void* logits, int logits_dtype, int tokens, int experts, int top_k, int iters,
+                        float epsilon, float temperature, int64_t* idx, void* weights, void* workspace,
+                        size_t workspace_bytes, void* stream);
 
 /*
  * Grouped expert GEMM over expert-contiguous rows (tcgen05 / TMEM, TMA-fed,

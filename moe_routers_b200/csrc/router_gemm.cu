@@ -109,35 +109,6 @@ __device__ __forceinline__ void key_insert(uint32_t (&keys)[KMAX], uint32_t c) {
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int32_t* status, int code) {
-#pragma unroll 1
-  for (int i = 0; i < 2048; ++i)
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  const unsigned long long limit = wait_limit_ns(status);
-  for (;;) {
-#pragma unroll 1
-    for (int i = 0; i < 256; ++i)
-      if (mbar_try_wait_cluster(bar, parity)) return true;
-    if (globaltimer_ns() - t0 > limit) {
-      record_error(status, kErrMbarTimeout | code);
-      return false;
-    }
-  }
-}
 // Shared memory of this CTA -> shared memory of a CTA of the cluster, completion counted in bytes on an
 // mbarrier of the destination CTA (both given as shared::cluster addresses); 16-byte granularity.
 __device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst_cluster, uint32_t src_cta, uint32_t bytes,

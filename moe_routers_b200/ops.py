@@ -273,6 +273,16 @@ def route_fused(x: torch.Tensor, w_router: torch.Tensor, top_k: int, *, skew_exp
 def sinkhorn(logits: torch.Tensor, top_k: int, *, iters: int = 10, epsilon: float = 1e-6,
              temperature: float = 1.0):
     """Sinkhorn-balanced top-k: (idx int32 [T,k], gates float32 [T,k])."""
+    return _sinkhorn(lib.moe_sinkhorn, torch.int32, torch.float32, logits, top_k, iters, epsilon, temperature)
+
+
+def sinkhorn_router(logits: torch.Tensor, top_k: int, *, iters: int = 10, epsilon: float = 1e-6,
+                    temperature: float = 1.0):
+    """The same as the router plug-in returns it: (idx int64 [T,k], weights [T,k] in the logits' type)."""
+    return _sinkhorn(lib.moe_sinkhorn_router, torch.int64, logits.dtype, logits, top_k, iters, epsilon, temperature)
+
+
+def _sinkhorn(entry, idx_dtype, gate_dtype, logits, top_k, iters, epsilon, temperature):
     _require_cuda(logits)
     if logits.dim() != 2:
         raise ValueError("SinkhornRouter expects logits of shape [tokens, experts]")
@@ -282,12 +292,11 @@ def sinkhorn(logits: torch.Tensor, top_k: int, *, iters: int = 10, epsilon: floa
     t, e = logits.shape
     dev = logits.device
     with torch.cuda.device(dev):
-        idx = torch.empty((t, top_k), dtype=torch.int32, device=dev)
-        gates = torch.empty((t, top_k), dtype=torch.float32, device=dev)
+        idx = torch.empty((t, top_k), dtype=idx_dtype, device=dev)
+        gates = torch.empty((t, top_k), dtype=gate_dtype, device=dev)
         ws = workspace(dev, t, e, top_k)
-        check(lib.moe_sinkhorn(logits.data_ptr(), _DTYPE_CODE[logits.dtype], t, e, int(top_k), int(iters),
-                               float(epsilon), float(temperature), idx.data_ptr(), gates.data_ptr(),
-                               ws.data_ptr(), ws.numel(), _stream()))
+        check(entry(logits.data_ptr(), _DTYPE_CODE[logits.dtype], t, e, int(top_k), int(iters), float(epsilon),
+                    float(temperature), idx.data_ptr(), gates.data_ptr(), ws.data_ptr(), ws.numel(), _stream()))
     return idx, gates
 
 

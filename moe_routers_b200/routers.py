@@ -62,6 +62,5 @@ class SinkhornRouter(RouterBase):
             raise ValueError("top_k must be > 0")
         if top_k > logits.size(1):
             raise ValueError("top_k must be <= n_experts")
-        idx, w = ops.sinkhorn(logits, int(top_k), iters=self.iters, epsilon=self.epsilon,
-                              temperature=self.temperature)
-        return idx.to(torch.int64), w.to(dtype=logits.dtype)
+        return ops.sinkhorn_router(logits, int(top_k), iters=self.iters, epsilon=self.epsilon,
+                                   temperature=self.temperature)
