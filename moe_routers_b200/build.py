@@ -1,4 +1,4 @@
-"""Build libmoe_b200.so in-tree with nvcc for sm_100a.
+"""Build libmoe_b200.so in-tree with nvcc for sm_100a, and the host extension _host.so with g++.
 
     python -m moe_routers_b200.build [--force] [--verbose]
 
@@ -10,15 +10,19 @@ or driver.
 from __future__ import annotations
 
 import glob
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libmoe_b200.so")
+HOST_SRC = os.path.join(CSRC, "host.cpp")
+HOST_PATH = os.path.join(PKG, "_host.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
 NVCC_FLAGS = [
@@ -48,8 +52,27 @@ def _stale() -> bool:
     return any(os.path.getmtime(p) > t for p in deps)
 
 
+def build_host(force: bool = False) -> str:
+    """Compile csrc/host.cpp against the installed torch's headers into the extension module _host.so."""
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= os.path.getmtime(HOST_SRC):
+        return HOST_PATH
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    includes = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+                sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=1"]
+    for path in includes:
+        cmd += ["-isystem", path]
+    cmd += [HOST_SRC, "-o", HOST_PATH, "-L", os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout)
+        raise RuntimeError(f"g++ failed on {HOST_SRC}")
+    return HOST_PATH
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compile every .cu under csrc/ into lib/libmoe_b200.so (no-op if fresh)."""
+    """Compile every .cu under csrc/ into lib/libmoe_b200.so and host.cpp into _host.so (no-op if fresh)."""
+    build_host(force)
     if not force and not _stale():
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)

@@ -38,6 +38,24 @@ int check_launch(const char* what) {
   return fail(MOE_ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(e));
 }
 
+cudaError_t grant_smem(const void* kernel, size_t bytes, SmemGrant& grant) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const bool kept = dev >= 0 && dev < 64;
+  if (kept && grant.bytes[dev].load(std::memory_order_relaxed) >= (int)bytes) return cudaSuccess;
+  int optin = 0;
+  cudaFuncAttributes attr;
+  e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, kernel);
+  if (e != cudaSuccess) return e;
+  const int most = optin - (int)attr.sharedSizeBytes;
+  const int ask = most >= (int)bytes ? most : (int)bytes;  // (more than there is: the call below refuses it)
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ask);
+  if (e == cudaSuccess && kept) grant.bytes[dev].store(ask, std::memory_order_relaxed);
+  return e;
+}
+
 // -1: not decided yet (the environment decides on first use), 0 / 1: off / on
 static std::atomic<int> g_pdl{-1};
 

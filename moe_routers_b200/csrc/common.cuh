@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 
@@ -67,6 +68,12 @@ void set_error(const char* fmt, ...);
 int fail(int code, const char* fmt, ...);
 int check_launch(const char* what);  // counts the launch when it succeeded
 void note_launch();                  // for launches checked by hand (cudaLaunchKernelEx)
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device.  The first call on a device grants
+// the kernel all that the device has, so that later launches of any size make no driver call.
+struct SmemGrant {
+  std::atomic<int> bytes[64];
+};
+cudaError_t grant_smem(const void* kernel, size_t bytes, SmemGrant& grant);
 bool pdl_enabled();                  // programmatic dependent launch between the route kernels
 
 __device__ __forceinline__ void record_error(int32_t* status, int code) {

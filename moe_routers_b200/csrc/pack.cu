@@ -337,7 +337,8 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
     if (nbuf >= kBulkIssuers) {
       const size_t smem = (size_t)nbuf * chunk + (size_t)nbuf * sizeof(uint64_t) +
                          (size_t)(2 * experts + 2 * kMaxTileRoutes) * sizeof(int32_t);
-      err = cudaFuncSetAttribute(pack_scatter_bulk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      static SmemGrant grant;
+      err = grant_smem(reinterpret_cast<const void*>(pack_scatter_bulk_kernel), smem, grant);
       if (err != cudaSuccess) return fail(MOE_ERR_LAUNCH, "pack_scatter_bulk_kernel: %s", cudaGetErrorString(err));
       cfg.gridDim = dim3(nt, 1, 1);
       cfg.dynamicSmemBytes = smem;

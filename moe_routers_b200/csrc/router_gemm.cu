@@ -561,7 +561,8 @@ int launch_router(const void* x, const void* w, int tokens, int d, int experts, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemGrant grants[4];  // one per KMAX
+  cudaError_t e = grant_smem(reinterpret_cast<const void*>(kernel), smem, grants[kmax == 8 ? 3 : kmax >> 1]);
   if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "router GEMM: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   e = cudaLaunchKernelEx(&cfg, kernel, tmap_x, tmap_w, p);
   if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "router_gemm_select_kernel: %s", cudaGetErrorString(e));

@@ -34,6 +34,15 @@ def _as_one(tensors: List[torch.Tensor]):
     return torch.cat([t.contiguous() for t in tensors], dim=0), False
 
 
+def _upload(offs: List[int], device: torch.device) -> torch.Tensor:
+    """int32 offsets on the device, through pinned memory: a copy from pageable memory waits for everything
+    enqueued before it.  (A captured copy would read the pinned buffer again at replay, so a capture takes the
+    pageable way, which it refuses.)"""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.tensor(offs, dtype=torch.int32, device=device)
+    return torch.tensor(offs, dtype=torch.int32).pin_memory().to(device, non_blocking=True)
+
+
 def grouped_ffn_forward(inputs: List[torch.Tensor], weights: List[torch.Tensor]) -> List[torch.Tensor]:
     if len(inputs) == 0:
         return []
@@ -55,6 +64,6 @@ def grouped_ffn_forward(inputs: List[torch.Tensor], weights: List[torch.Tensor])
     offs = [0]
     for c in counts:
         offs.append(offs[-1] + c)
-    offsets = torch.tensor(offs, dtype=torch.int32, device=a_all.device)
+    offsets = _upload(offs, a_all.device)
     out = ops.grouped_gemm(a_all, w_all.reshape(len(weights), k_dim, n_dim), offsets, layout="kn")
     return list(torch.split(out, counts, dim=0))

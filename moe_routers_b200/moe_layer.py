@@ -20,6 +20,7 @@ from typing import Optional
 import torch
 
 from . import ops
+from ._host import weight_state
 from .metrics import (ExpertUsageMetrics, MoEMetrics, PerformanceEfficiencyMetrics, RoutingBehaviorMetrics,
                       aux_load_balance_loss, avg_unique_experts_per_token, mean_topk_probability_from_logits,
                       normalized_entropy, output_distribution_stats, routing_entropy_from_distribution,
@@ -74,8 +75,10 @@ class MoELayer(torch.nn.Module):
 
     def _stacked_weights(self):
         """[E, 2h, d] (gate rows, then up rows) and [E, d, h], rebuilt when a parameter changes."""
-        params = [p for ex in self.experts for p in (ex.w1.weight, ex.w3.weight, ex.w2.weight)]
-        key = tuple((p.data_ptr(), p._version) for p in params)
+        key = weight_state(self.experts._modules, ("w1", "w3", "w2"))
+        if key is None:  # some weight is not a plain parameter
+            params = [p for ex in self.experts for p in (ex.w1.weight, ex.w3.weight, ex.w2.weight)]
+            key = tuple((p.data_ptr(), p._version) for p in params)
         if self._stacked is None or key != self._stacked_key:
             w13 = torch.stack([torch.cat([ex.w1.weight, ex.w3.weight], dim=0) for ex in self.experts]).contiguous()
             w2 = torch.stack([ex.w2.weight for ex in self.experts]).contiguous()

@@ -8,11 +8,13 @@ rejected.
 """
 from __future__ import annotations
 
+import contextlib
 from typing import Optional
 
 import torch
 
 from . import _lib
+from ._host import empties
 from ._lib import check, lib
 
 _DTYPE_CODE = {torch.float16: _lib.MOE_F16, torch.bfloat16: _lib.MOE_BF16, torch.float32: _lib.MOE_F32}
@@ -20,8 +22,19 @@ _DTYPE_CODE = {torch.float16: _lib.MOE_F16, torch.bfloat16: _lib.MOE_BF16, torch
 _workspaces: dict = {}
 
 
+# The current stream's handle and the current device, without building a Stream or Device object.
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_current_device = torch._C._cuda_getDevice
+_SAME_DEVICE = contextlib.nullcontext()
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
+
+
+def _on(index: int):
+    """Makes CUDA device `index` current for a `with` block (nothing to do where it is)."""
+    return _SAME_DEVICE if index == _current_device() else torch.cuda.device(index)
 
 
 def _require_cuda(*tensors: torch.Tensor) -> None:
@@ -32,12 +45,15 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
 
 def workspace(device: torch.device, tokens: int, experts: int, top_k: int) -> torch.Tensor:
     """Per (device, stream) scratch buffer, grown on demand and initialised once."""
-    need = int(lib.moe_workspace_bytes(int(tokens), int(experts), int(top_k)))
-    need = max(need, 1 << 16)
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
+    return _workspace(device.index if device.index is not None else torch.cuda.current_device(), tokens, experts, top_k)
+
+
+def _workspace(index: int, tokens: int, experts: int, top_k: int) -> torch.Tensor:
+    need = max(lib.moe_workspace_bytes(int(tokens), int(experts), int(top_k)), 1 << 16)
+    key = (index, _stream())
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < need:
-        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=device)
+        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", index))
         check(lib.moe_workspace_init(ws.data_ptr(), ws.numel(), _stream()))
         _workspaces[key] = ws
     return ws
@@ -63,12 +79,22 @@ def topk_select(logits: torch.Tensor, top_k: int):
         raise RuntimeError("logits must be fp16/bf16/fp32")
     logits = logits.contiguous()
     t, e = logits.shape
-    with torch.cuda.device(logits.device):
-        idx = torch.empty((t, top_k), dtype=torch.int32, device=logits.device)
-        gates = torch.empty((t, top_k), dtype=torch.float32, device=logits.device)
+    dev = logits.get_device()
+    with _on(dev):
+        idx, gates = empties(dev, ((torch.int32, t, top_k), (torch.float32, t, top_k)))
         check(lib.moe_topk_select(logits.data_ptr(), _DTYPE_CODE[logits.dtype], t, e, int(top_k),
                                   idx.data_ptr(), gates.data_ptr(), _stream()))
     return idx, gates
+
+
+def _map_specs(t: int, experts: int, k: int):
+    """counts, offsets, row_route, route_row"""
+    return (torch.int32, experts), (torch.int32, experts + 1), (torch.int32, t * k), (torch.int32, t * k)
+
+
+def _route_specs(t: int, d: int, experts: int, k: int, dtype: torch.dtype):
+    """idx, gates, packed, counts, offsets, row_route, route_row"""
+    return ((torch.int32, t, k), (torch.float32, t, k), (dtype, t * k, d)) + _map_specs(t, experts, k)
 
 
 def pack(x: torch.Tensor, idx: torch.Tensor, experts: int, *, copy_rows: bool = True):
@@ -82,14 +108,11 @@ def pack(x: torch.Tensor, idx: torch.Tensor, experts: int, *, copy_rows: bool = 
     idx = idx.to(torch.int32).contiguous()
     t, d = x.shape
     k = idx.size(1)
-    dev = x.device
-    with torch.cuda.device(dev):
-        counts = torch.empty(experts, dtype=torch.int32, device=dev)
-        offsets = torch.empty(experts + 1, dtype=torch.int32, device=dev)
-        packed = torch.empty((t * k, d), dtype=x.dtype, device=dev) if copy_rows else None
-        row_route = torch.empty(t * k, dtype=torch.int32, device=dev)
-        route_row = torch.empty(t * k, dtype=torch.int32, device=dev)
-        ws = workspace(dev, t, experts, k)
+    dev = x.get_device()
+    with _on(dev):
+        counts, offsets, row_route, route_row = empties(dev, _map_specs(t, experts, k))
+        packed = empties(dev, ((x.dtype, t * k, d),))[0] if copy_rows else None
+        ws = _workspace(dev, t, experts, k)
         check(lib.moe_pack(x.data_ptr(), x.element_size(), idx.data_ptr(), t, d, int(experts), k,
                            counts.data_ptr(), offsets.data_ptr(),
                            packed.data_ptr() if packed is not None else None,
@@ -107,7 +130,7 @@ def pack_scatter(x: torch.Tensor, experts: int, out: dict) -> dict:
     _require_cuda(x)
     t, d = x.shape
     k = out["idx"].size(1)
-    with torch.cuda.device(x.device):
+    with _on(x.get_device()):
         ws = out["workspace"]
         check(lib.moe_pack_scatter(x.data_ptr(), x.element_size(), out["idx"].data_ptr(), t, d, int(experts), k,
                                    out["counts"].data_ptr(), out["offsets"].data_ptr(), out["packed"].data_ptr(),
@@ -126,13 +149,11 @@ def route_plan(x: torch.Tensor, idx: torch.Tensor, experts: int, *, hist_ready: 
     idx = idx.to(torch.int32).contiguous()
     t, d = x.shape
     k = idx.size(1)
-    dev = x.device
-    with torch.cuda.device(dev):
-        o = dict(idx=idx, counts=torch.empty(experts, dtype=torch.int32, device=dev),
-                 offsets=torch.empty(experts + 1, dtype=torch.int32, device=dev),
-                 row_route=torch.empty(t * k, dtype=torch.int32, device=dev),
-                 route_row=torch.empty(t * k, dtype=torch.int32, device=dev))
-        ws = o["workspace"] = workspace(dev, t, experts, k)
+    dev = x.get_device()
+    with _on(dev):
+        counts, offsets, row_route, route_row = empties(dev, _map_specs(t, experts, k))
+        ws = _workspace(dev, t, experts, k)
+        o = dict(idx=idx, counts=counts, offsets=offsets, row_route=row_route, route_row=route_row, workspace=ws)
         fn = lib.moe_pack_scatter if hist_ready else lib.moe_pack
         check(fn(x.data_ptr(), x.element_size(), idx.data_ptr(), t, d, int(experts), k, o["counts"].data_ptr(),
                  o["offsets"].data_ptr(), None, o["row_route"].data_ptr(), o["route_row"].data_ptr(),
@@ -152,7 +173,7 @@ def pack_scatter_to(x: torch.Tensor, experts: int, plan: dict, seg_base: torch.T
     t, d = x.shape
     k = plan["idx"].size(1)
     ws = plan["workspace"]
-    with torch.cuda.device(x.device):
+    with _on(x.get_device()):
         check(lib.moe_pack_scatter_to(x.data_ptr(), x.element_size(), plan["idx"].data_ptr(), t, d, int(experts), k,
                                       plan["counts"].data_ptr(), plan["offsets"].data_ptr(), seg_base.data_ptr(),
                                       plan["row_route"].data_ptr(), plan["route_row"].data_ptr(), ws.data_ptr(),
@@ -170,18 +191,14 @@ def fused_select(logits: torch.Tensor, x: torch.Tensor, experts: int, top_k: int
     logits = logits.contiguous()
     x = x.contiguous()
     t, d = x.shape
-    dev = x.device
-    with torch.cuda.device(dev):
+    dev = x.get_device()
+    with _on(dev):
         if out is None:
-            out = (torch.empty((t, top_k), dtype=torch.int32, device=dev),
-                   torch.empty((t, top_k), dtype=torch.float32, device=dev),
-                   torch.empty(experts, dtype=torch.int32, device=dev),
-                   torch.empty(experts + 1, dtype=torch.int32, device=dev),
-                   torch.empty((t * top_k, d), dtype=x.dtype, device=dev),
-                   torch.empty(t * top_k, dtype=torch.int32, device=dev),
-                   torch.empty(t * top_k, dtype=torch.int32, device=dev))
-        idx, gates, counts, offsets, packed, row_route, route_row = out
-        ws = workspace(dev, t, experts, top_k)
+            idx, gates, packed, counts, offsets, row_route, route_row = empties(dev, _route_specs(t, d, experts, top_k, x.dtype))
+            out = (idx, gates, counts, offsets, packed, row_route, route_row)
+        else:
+            idx, gates, counts, offsets, packed, row_route, route_row = out
+        ws = _workspace(dev, t, experts, top_k)
         check(lib.moe_fused_select(logits.data_ptr(), _DTYPE_CODE[logits.dtype], x.data_ptr(), x.element_size(), t, d,
                                    int(experts), int(top_k), idx.data_ptr(), gates.data_ptr(), counts.data_ptr(),
                                    offsets.data_ptr(), packed.data_ptr(), row_route.data_ptr(), route_row.data_ptr(),
@@ -199,8 +216,9 @@ def combine(y: torch.Tensor, gates: torch.Tensor, route_row: torch.Tensor, top_k
     route_row = route_row.to(torch.int32).contiguous()
     rows, d = y.shape
     t = rows // top_k
-    with torch.cuda.device(y.device):
-        out = torch.empty((t, d), dtype=y.dtype, device=y.device)
+    dev = y.get_device()
+    with _on(dev):
+        out, = empties(dev, ((y.dtype, t, d),))
         check(lib.moe_combine(y.data_ptr(), _DTYPE_CODE[y.dtype], gates.data_ptr(), route_row.data_ptr(),
                               t, d, int(top_k), out.data_ptr(), _stream()))
     return out
@@ -216,12 +234,11 @@ def router_gemm_select(x: torch.Tensor, w_router: torch.Tensor, top_k: int, *, s
     w_router = w_router.contiguous()
     t, d = x.shape
     e = w_router.size(0)
-    dev = x.device
-    with torch.cuda.device(dev):
-        idx = torch.empty((t, top_k), dtype=torch.int32, device=dev)
-        gates = torch.empty((t, top_k), dtype=torch.float32, device=dev)
-        logits = torch.empty((t, e), dtype=torch.float32, device=dev) if return_logits else None
-        ws = workspace(dev, t, e, top_k)
+    dev = x.get_device()
+    with _on(dev):
+        idx, gates = empties(dev, ((torch.int32, t, top_k), (torch.float32, t, top_k)))
+        logits = empties(dev, ((torch.float32, t, e),))[0] if return_logits else None
+        ws = _workspace(dev, t, e, top_k)
         check(lib.moe_router_gemm_select(x.data_ptr(), w_router.data_ptr(), _DTYPE_CODE[x.dtype], t, d, e, int(top_k),
                                          int(skew_experts), float(skew_bias), idx.data_ptr(),
                                          gates.data_ptr(), logits.data_ptr() if return_logits else None,
@@ -246,20 +263,16 @@ def route_fused(x: torch.Tensor, w_router: torch.Tensor, top_k: int, *, skew_exp
     w_router = w_router.contiguous()
     t, d = x.shape
     e = w_router.size(0)
-    dev = x.device
-    with torch.cuda.device(dev):
+    dev = x.get_device()
+    with _on(dev):
         o = out if out is not None else {}
         if "idx" not in o:
-            o["idx"] = torch.empty((t, top_k), dtype=torch.int32, device=dev)
-            o["gates"] = torch.empty((t, top_k), dtype=torch.float32, device=dev)
-            o["counts"] = torch.empty(e, dtype=torch.int32, device=dev)
-            o["offsets"] = torch.empty(e + 1, dtype=torch.int32, device=dev)
-            o["packed"] = torch.empty((t * top_k, d), dtype=x.dtype, device=dev)
-            o["row_route"] = torch.empty(t * top_k, dtype=torch.int32, device=dev)
-            o["route_row"] = torch.empty(t * top_k, dtype=torch.int32, device=dev)
+            idx, gates, packed, counts, offsets, row_route, route_row = empties(dev, _route_specs(t, d, e, top_k, x.dtype))
+            o.update(idx=idx, gates=gates, counts=counts, offsets=offsets, packed=packed, row_route=row_route,
+                     route_row=route_row)
         if return_logits and "logits" not in o:
-            o["logits"] = torch.empty((t, e), dtype=torch.float32, device=dev)
-        ws = o["workspace"] = workspace(dev, t, e, top_k)
+            o["logits"], = empties(dev, ((torch.float32, t, e),))
+        ws = o["workspace"] = _workspace(dev, t, e, top_k)
         check(lib.moe_route_fused(x.data_ptr(), w_router.data_ptr(), _DTYPE_CODE[x.dtype], t, d, e, int(top_k),
                                   int(skew_experts), float(skew_bias), o["idx"].data_ptr(),
                                   o["gates"].data_ptr(), o["counts"].data_ptr(), o["offsets"].data_ptr(),
@@ -290,11 +303,10 @@ def _sinkhorn(entry, idx_dtype, gate_dtype, logits, top_k, iters, epsilon, tempe
         raise RuntimeError("logits must be fp16/bf16/fp32")
     logits = logits.contiguous()
     t, e = logits.shape
-    dev = logits.device
-    with torch.cuda.device(dev):
-        idx = torch.empty((t, top_k), dtype=idx_dtype, device=dev)
-        gates = torch.empty((t, top_k), dtype=gate_dtype, device=dev)
-        ws = workspace(dev, t, e, top_k)
+    dev = logits.get_device()
+    with _on(dev):
+        idx, gates = empties(dev, ((idx_dtype, t, top_k), (gate_dtype, t, top_k)))
+        ws = _workspace(dev, t, e, top_k)
         check(entry(logits.data_ptr(), _DTYPE_CODE[logits.dtype], t, e, int(top_k), int(iters), float(epsilon),
                     float(temperature), idx.data_ptr(), gates.data_ptr(), ws.data_ptr(), ws.numel(), _stream()))
     return idx, gates
@@ -335,9 +347,9 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, *, lay
         raise RuntimeError("grouped_gemm: inner dimensions differ")
     act = _ACT[activation]
     n_out = n_w // 2 if act == _lib.MOE_ACT_SWIGLU else n_w
-    dev = a.device
-    with torch.cuda.device(dev):
-        ws = workspace(dev, 1, e, 1)
+    dev = a.get_device()
+    with _on(dev):
+        ws = _workspace(dev, 1, e, 1)
         rs = row_scale.to(torch.float32).contiguous() if row_scale is not None else None
         if out_rows is not None:
             if out_rows.dtype != torch.int64 or not out_rows.is_cuda or out_rows.numel() < rows:
@@ -350,7 +362,7 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, *, lay
                                             _DTYPE_CODE[a.dtype], int(sm_margin), ws.data_ptr(), ws.numel(),
                                             _stream()))
             return out_rows
-        c = out if out is not None else torch.empty((rows, n_out), dtype=a.dtype, device=dev)
+        c = out if out is not None else empties(dev, ((a.dtype, rows, n_out),))[0]
         check(lib.moe_grouped_gemm(a.data_ptr(), w.data_ptr(), c.data_ptr(), offsets.data_ptr(), e, rows,
                                    k_dim, n_out, _lib.MOE_W_NK if layout == "nk" else _lib.MOE_W_KN,
                                    w.stride(0), act, rs.data_ptr() if rs is not None else None,
