@@ -154,23 +154,26 @@ pack_scatter_kernel(const char* __restrict__ x, const int32_t* __restrict__ idx,
 }
 
 // ---------------------------------------------------------------------------
-// Bulk-copy scatter (rows a multiple of 16 bytes, 16-byte aligned bases): one CTA per tile of 32
-// tokens.  Token rows are staged through a ring of shared-memory buffers by the TMA engine:
+// Bulk-copy scatter (rows a multiple of 16 bytes, 16-byte aligned bases): `split` CTAs per tile of 32
+// tokens, each of which ranks the whole tile and copies its share of the tokens.  Token rows are staged through a ring of shared-memory buffers by the TMA engine:
 //   global --cp.async.bulk--> shared (mbarrier complete_tx) --cp.async.bulk--> top_k global rows.
 // A row longer than kChunkBytes is moved in chunks.  Lane 0 of each of the 8 warps drives every
 // 8th item (item = row chunk); buffer (item % NBUF) with NBUF a multiple of 8, so a buffer is only
 // ever reused by the thread that filled it, after that thread's stores have finished reading it.
 // The first loads are issued before the destinations are known: they do not depend on the routing.
 constexpr int kBulkIssuers = kScatterThreads / 32;
+constexpr int kSms = 148;
+constexpr int kMaxSplit = 8;     // CTAs per tile
+constexpr int kMinChunk = 2048;
 
-__global__ void __launch_bounds__(kScatterThreads, 1)
+__global__ void __launch_bounds__(kScatterThreads, 2)
 pack_scatter_bulk_kernel(const char* __restrict__ x, const int32_t* __restrict__ idx,
                          const int32_t* __restrict__ tile_hist, const int32_t* __restrict__ tile_base,
                          int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
                          char* __restrict__ packed, int32_t* __restrict__ row_route,
                          int32_t* __restrict__ route_row, int tokens, size_t row_bytes, int experts,
-                         int top_k, int num_tiles, int nbuf, int chunk_bytes, int early_rows, int32_t* status,
-                         char* const* __restrict__ seg_base) {
+                         int top_k, int num_tiles, int split, int nbuf, int chunk_bytes, int early_rows,
+                         int32_t* status, char* const* __restrict__ seg_base) {
   extern __shared__ __align__(128) uint8_t s_raw[];
   uint8_t* s_buf = s_raw;                                                        // [nbuf][chunk_bytes]
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_buf + (size_t)nbuf * chunk_bytes);  // [nbuf]
@@ -179,13 +182,16 @@ pack_scatter_bulk_kernel(const char* __restrict__ x, const int32_t* __restrict__
   int32_t* s_dst = s_total + experts;                                            // [kMaxTileRoutes]
   int32_t* s_exp = s_dst + kMaxTileRoutes;                                       // [kMaxTileRoutes], seg_base only
 
-  const int tile = blockIdx.x;
+  const int tile = blockIdx.x / split;
+  const int part = blockIdx.x % split;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int t0 = tile * kTileTokens;
   const int tile_tokens = min(kTileTokens, tokens - t0);
+  const int lt0 = part * (kTileTokens / split);  // this CTA's tokens of the tile
+  const int part_tokens = max(0, min(kTileTokens / split, tile_tokens - lt0));
   const int chunks = (int)((row_bytes + chunk_bytes - 1) / chunk_bytes);
-  const int items = (packed != nullptr || seg_base != nullptr) ? tile_tokens * chunks : 0;
+  const int items = (packed != nullptr || seg_base != nullptr) ? part_tokens * chunks : 0;
   const int depth = nbuf / kBulkIssuers;  // buffers owned by each issuing thread
 
   // a kernel launched behind this one with programmatic stream serialisation (the next route's
@@ -206,7 +212,7 @@ pack_scatter_bulk_kernel(const char* __restrict__ x, const int32_t* __restrict__
     const int row = chunks == 1 ? it : it / chunks, ch = chunks == 1 ? 0 : it % chunks;
     const size_t ofs = (size_t)ch * chunk_bytes;
     bytes = (uint32_t)min((size_t)chunk_bytes, row_bytes - ofs);
-    return x + (size_t)(t0 + row) * row_bytes + ofs;
+    return x + (size_t)(t0 + lt0 + row) * row_bytes + ofs;
   };
   // The rows may be read ahead of the dependency wait only where the caller knows that no kernel still
   // running can be writing them.
@@ -225,7 +231,7 @@ pack_scatter_bulk_kernel(const char* __restrict__ x, const int32_t* __restrict__
 
   asm volatile("griddepcontrol.wait;" ::: "memory");
   tile_destinations(idx, tile_hist, tile_base, counts, offsets, row_route, route_row, tile, t0,
-                    tile_tokens * top_k, experts, top_k, num_tiles, blockIdx.x == 0, true, s_base, s_total,
+                    tile_tokens * top_k, experts, top_k, num_tiles, blockIdx.x == 0, part == 0, s_base, s_total,
                     s_dst, status, seg_base != nullptr ? s_exp : nullptr);
 
   if (lane == 0) {
@@ -239,7 +245,7 @@ pack_scatter_bulk_kernel(const char* __restrict__ x, const int32_t* __restrict__
       ok = sm100::mbar_wait(bar0 + 8u * b, par, status, 8);
       if (!ok) break;
       if (++slot == depth) { slot = 0; par ^= 1u; }
-      const int row = chunks == 1 ? it : it / chunks, ch = chunks == 1 ? 0 : it % chunks;
+      const int row = lt0 + (chunks == 1 ? it : it / chunks), ch = chunks == 1 ? 0 : it % chunks;
       uint32_t bytes;
       (void)item_src(it, bytes);
       for (int j = 0; j < top_k; ++j) {
@@ -326,11 +332,28 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
 
   char* const* sb = reinterpret_cast<char* const*>(seg_base);
   if ((align & 15) == 0 && (packed != nullptr || sb != nullptr)) {
-    const int chunk = (int)(row_bytes < (size_t)kChunkBytes ? row_bytes : (size_t)kChunkBytes);
-    const int chunks = (int)((row_bytes + chunk - 1) / chunk);
+    // With fewer tiles than half the SMs a tile is copied by up to 8 CTAs; where there are between one and two
+    // CTAs per SM the ring is sized for two, so that they run as one wave.  Otherwise a CTA takes a whole tile
+    // and the SM's shared memory (a second resident CTA, or a split with 75..148 tiles, was 1..10 % slower).
+    // Device time of the route (router + scatter), before -> after: 16 x 4096, E 64, k 2: 15.7 -> 12.6 us;
+    // 600: 21.5 -> 15.1; 1024, E 128, k 4: 34.5 -> 22.5; 2049 x 2048, E 256, k 8: 48.1 -> 41.2;
+    // 8192 x 2048, E 32, k 4: 46.2 -> 42.7 us.
+    int split = 1;
+    if (nt * 2 <= kSms)
+      while (split < kMaxSplit && nt * split < kSms) split *= 2;
+    const int per_cta = kTileTokens / split;
+    int chunk = (int)(row_bytes < (size_t)kChunkBytes ? row_bytes : (size_t)kChunkBytes);
+    int chunks = (int)((row_bytes + chunk - 1) / chunk);
+    // rows in pieces where a CTA would have fewer items than issuing threads
+    while (per_cta * chunks < kBulkIssuers && chunk >= 2 * kMinChunk) {
+      chunk = ((chunk / 2) + 15) & ~15;
+      chunks = (int)((row_bytes + chunk - 1) / chunk);
+    }
     const size_t fixed = (size_t)(2 * experts + 2 * kMaxTileRoutes) * sizeof(int32_t) + 64 * sizeof(uint64_t) + 128;
-    int nbuf = (int)((227 * 1024 - fixed) / chunk);
-    const int want = ((kTileTokens * chunks + kBulkIssuers - 1) / kBulkIssuers) * kBulkIssuers;
+    const int want = ((per_cta * chunks + kBulkIssuers - 1) / kBulkIssuers) * kBulkIssuers;
+    int nbuf = 0;
+    for (int resident = nt * split > kSms && nt * split <= 2 * kSms ? 2 : 1; resident >= 1 && nbuf < kBulkIssuers; --resident)
+      nbuf = (int)((227 * 1024 / resident - 1024 - fixed) / chunk);
     if (nbuf > want) nbuf = want;
     if (nbuf > 64) nbuf = 64;
     nbuf = (nbuf / kBulkIssuers) * kBulkIssuers;
@@ -340,10 +363,10 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
       static SmemGrant grant;
       err = grant_smem(reinterpret_cast<const void*>(pack_scatter_bulk_kernel), smem, grant);
       if (err != cudaSuccess) return fail(MOE_ERR_LAUNCH, "pack_scatter_bulk_kernel: %s", cudaGetErrorString(err));
-      cfg.gridDim = dim3(nt, 1, 1);
+      cfg.gridDim = dim3(nt * split, 1, 1);
       cfg.dynamicSmemBytes = smem;
       err = cudaLaunchKernelEx(&cfg, pack_scatter_bulk_kernel, xs, idx, th, tile_base, counts, offsets, ps,
-                               row_route, route_row, tokens, row_bytes, experts, top_k, nt, nbuf, chunk,
+                               row_route, route_row, tokens, row_bytes, experts, top_k, nt, split, nbuf, chunk,
                                early_rows ? 1 : 0, st, sb);
       if (err != cudaSuccess) return fail(MOE_ERR_LAUNCH, "pack_scatter_bulk_kernel: %s", cudaGetErrorString(err));
       note_launch();

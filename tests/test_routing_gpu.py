@@ -222,3 +222,23 @@ def test_fused_select_equals_select_then_pack(ops, t, d, e, k, dtype):
     assert torch.equal(counts, c2) and torch.equal(offsets, o2) and torch.equal(packed, p2)
     assert torch.equal(row_route, rr2) and torch.equal(route_row, ir2)
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("t", [1, 31, 32, 33, 65, 592, 593, 2336, 2368, 2369, 4736, 4737, 4800, 9472, 9473])
+@pytest.mark.parametrize("d,dtype,k", [(8, torch.float16, 2), (1032, torch.bfloat16, 3), (4104, torch.float32, 1)])
+def test_scatter_split_edges(t, d, dtype, k):
+    """Tiles copied by 1, 2, 4 or 8 CTAs and one or two CTAs per SM: the token counts at which that changes, with
+    rows of one, several and uneven pieces."""
+    from moe_routers_b200 import ops
+
+    g = torch.Generator().manual_seed(t + d)
+    e = 40
+    x = torch.randn(t, d, generator=g).to(dtype).cuda()
+    idx = torch.stack([torch.randperm(e, generator=g)[:k] for _ in range(t)]).int().cuda()
+    counts, offsets, packed, row_route, route_row = ops.pack(x, idx, e)
+    order = torch.sort(idx.flatten().long(), stable=True).indices
+    assert torch.equal(row_route.long(), order)
+    assert torch.equal(packed, x[order // k])
+    assert torch.equal(counts.long(), torch.bincount(idx.flatten().long(), minlength=e))
+    assert torch.equal(route_row.long()[order], torch.arange(t * k, device="cuda"))
+    assert ops.read_status() == 0
