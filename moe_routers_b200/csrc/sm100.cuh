@@ -170,51 +170,60 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc], fp16/bf16 inputs, fp32 accumulate.
+// D[tmem] (+)= A[smem desc] * B[smem desc], fp16/bf16 inputs, fp32 accumulate.  Called by a whole warp with the
+// same operands in every lane; one elected lane issues.  The election belongs to the instruction: eight MMAs then
+// take their warp 190 cycles to issue; with a lane chosen beforehand (a predicate from the lane number, or a
+// branch) the compiler cannot know that the operands are uniform, and the same eight take 690 or 510 cycles
+// whatever N is.
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, q;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "elect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on an mbarrier once every previously issued MMA of this thread has
+// Arrive on an mbarrier once every MMA that this warp has issued has
 // completed (implies tcgen05.fence::before_thread_sync).
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "elect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar)
+      : "memory");
 }
-// The CTA-pair forms (`cta_group::2`, issued by the one thread of a warp of the pair's even CTA that has
-// `issue` set): D is 256 x N, rows
+// The CTA-pair forms (`cta_group::2`), called by a whole warp of the pair's even CTA: D is 256 x N, rows
 // 0..127 accumulate in this CTA's TMEM and rows 128..255 in the other CTA's at the same TMEM address;
 // each CTA's shared memory holds its own 128 rows of A and its own N/2 columns of B at the same
 // offsets, which is what the descriptors (built from this CTA's addresses) name.
 __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate, uint32_t issue) {
+                                              uint32_t accumulate) {
   asm volatile(
       "{\n"
       ".reg .pred p, q;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "setp.ne.b32 q, %5, 0;\n"
+      "elect.sync _|q, 0xffffffff;\n"
       "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // Arrive on the mbarrier at this shared-memory offset in every CTA of `cta_mask` once the pair's MMAs
-// that this thread has issued have completed (a barrier signal, not a data copy).
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t cta_mask, uint32_t issue) {
+// that this warp has issued have completed (a barrier signal, not a data copy).
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t cta_mask) {
   asm volatile(
       "{\n"
       ".reg .pred q;\n"
-      "setp.ne.b32 q, %2, 0;\n"
+      "elect.sync _|q, 0xffffffff;\n"
       "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
       "}\n" ::"r"(bar),
-      "h"(cta_mask), "r"(issue)
+      "h"(cta_mask)
       : "memory");
 }
 // 32 lanes x 16 consecutive fp32 columns: thread i of the warp gets lane
