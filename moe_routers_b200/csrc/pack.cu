@@ -54,6 +54,10 @@ __global__ void __launch_bounds__(256)
 pack_scan_kernel(const int32_t* __restrict__ tile_hist, int32_t* __restrict__ tile_base,
                  int32_t* __restrict__ counts, int num_tiles, int experts) {
   __shared__ int32_t s_warp[8];
+  // launched with programmatic stream serialisation; the scatter behind it may start only now, since it
+  // fetches token rows ahead of its own wait
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int e = blockIdx.x;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -302,12 +306,27 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
     pack_zero_kernel<<<(experts + 256) / 256, 256, 0, s>>>(counts, offsets, experts);
     return check_launch("pack_zero_kernel");
   }
+  // Programmatic dependent launch: the scan and the scatter may become resident while the kernel in front of
+  // them is still running; the scatter prefetches token rows and then blocks in griddepcontrol.wait.
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kScatterThreads, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cudaError_t err;
+
   const int32_t* tile_base = nullptr;
   if (ws.num_tiles > kFusedPrefixTiles) {
-    pack_scan_kernel<<<experts, 256, 0, s>>>(ws.tile_hist, ws.tile_base, counts, ws.num_tiles, experts);
-    const int rc = check_launch("pack_scan_kernel");
-    if (rc != MOE_OK) return rc;
+    cfg.gridDim = dim3(experts, 1, 1);
+    err = cudaLaunchKernelEx(&cfg, pack_scan_kernel, static_cast<const int32_t*>(ws.tile_hist), ws.tile_base, counts,
+                             ws.num_tiles, experts);
+    if (err != cudaSuccess) return fail(MOE_ERR_LAUNCH, "pack_scan_kernel: %s", cudaGetErrorString(err));
+    note_launch();
     tile_base = ws.tile_base;
+    early_rows = true;  // the scan has waited for everything in front of it and writes no row
   }
   const size_t row_bytes = (size_t)d * elem_bytes;
   const uintptr_t align = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed) | row_bytes;
@@ -316,19 +335,6 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
   const int32_t* th = ws.tile_hist;
   int32_t* st = ws.status;
   const int nt = ws.num_tiles;
-
-  // Programmatic dependent launch: the scatter may become resident while the producer of the tile
-  // histograms (router GEMM or histogram kernel) is still running; it prefetches token rows and
-  // then blocks in griddepcontrol.wait until that kernel has completed.
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kScatterThreads, 1, 1);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (tile_base == nullptr && pdl_enabled()) ? 1 : 0;
-  cudaError_t err;
 
   char* const* sb = reinterpret_cast<char* const*>(seg_base);
   if ((align & 15) == 0 && (packed != nullptr || sb != nullptr)) {
