@@ -57,7 +57,9 @@ struct RouterParams {
   int bf16;  // 0: fp16 tokens / weights / logits, 1: bf16
   int epad;  // experts rounded up to the UMMA N granule (16); padded logit columns are never selected
   int kblocks, splitk, stages, tmem_cols, num_tiles;
+  int ring_bytes;     // pipeline stages (and what reuses them)
   int stage_in_ring;  // the exchange's transpose tiles reuse the pipeline stages
+  int part_in_ring;   // so do the partial tiles, once every CTA of the cluster has finished its MMAs
   int bulk_push;      // the exchange moves a warp's 32 x (E + 4) quarter with one bulk copy (E == 64 only)
   int prefetch_x;     // request this CTA's token boxes into L2 before the dependency wait
   int nacc;  // MMA-issuing warps = TMEM accumulators (1 or 2; at most the stage count)
@@ -259,14 +261,18 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
   const int EP = E + 4;  // padded row of a partial tile: conflict-free 128-bit accesses
   uint8_t* sA = smem;
   uint8_t* sB = sA + (size_t)p.stages * kABytes;
-  float* s_partial = reinterpret_cast<float*>(sB + (size_t)p.stages * b_bytes);  // [4][32][EP]
-  // transpose tiles of the exchange [4 warps][32][kChunk + 4]: the pipeline stages themselves once the
-  // last MMA has read them (the usual case), else a region of their own behind the partial tiles
-  float* s_own_stage = s_partial + (size_t)4 * 32 * EP;
-  float* s_stage = p.stage_in_ring ? reinterpret_cast<float*>(smem) : s_own_stage;
-  int32_t* s_hist = reinterpret_cast<int32_t*>(s_own_stage + (p.stage_in_ring ? 0 : kEpiWarps * 32 * (kChunk + 4)));  // [4][E]
-  uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_hist + 4 * E);  // full[], empty[], tmem_full, part_full
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + 2 * kMaxStages + 2);
+  // partial tiles [4][32][EP] behind the ring, or at its start; transpose tiles of the exchange [4 warps][32]
+  // [kChunk + 4]: the ring itself once the last MMA has read it (the usual case; behind the partial tiles where
+  // those are in the ring too), else a region of their own
+  float* s_tail = reinterpret_cast<float*>(smem + p.ring_bytes);
+  float* s_partial = p.part_in_ring ? reinterpret_cast<float*>(smem) : s_tail;
+  if (!p.part_in_ring) s_tail += (size_t)4 * 32 * EP;
+  float* s_stage = p.part_in_ring ? s_partial + (size_t)4 * 32 * EP
+                                  : (p.stage_in_ring ? reinterpret_cast<float*>(smem) : s_tail);
+  if (!p.stage_in_ring) s_tail += kEpiWarps * 32 * (kChunk + 4);
+  int32_t* s_hist = reinterpret_cast<int32_t*>(s_tail);  // [4][E]
+  uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_hist + 4 * E);  // full[], empty[], tmem_full, part_full, part_go
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + 2 * kMaxStages + 3);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -284,6 +290,7 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
   const uint32_t empty0 = smem_u32(s_bar + kMaxStages);
   const uint32_t tmem_full = smem_u32(s_bar + 2 * kMaxStages);
   const uint32_t part_full = smem_u32(s_bar + 2 * kMaxStages + 1);
+  const uint32_t part_go = smem_u32(s_bar + 2 * kMaxStages + 2);  // every CTA's ring is free (part_in_ring)
 
   // One barrier per thread (the prologue is on the critical path of the first copy); the descriptor
   // fetches start at once, from a warp that initialises nothing.
@@ -298,10 +305,11 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
     if (p.prefetch_x)
       for (int it = 0; it < nkb; ++it) tma_prefetch_l2_2d(&tmap_x, (kb0 + it) * kBlockK, block * kBlockTokens);
   }
-  if ((int)threadIdx.x < 2 * p.stages + 2) {
+  if ((int)threadIdx.x < 2 * p.stages + 3) {
     const int t = (int)threadIdx.x;
     if (t < p.stages) mbar_init(full0 + 8 * t, 1);
     else if (t < 2 * p.stages) mbar_init(empty0 + 8 * (t - p.stages), 1);
+    else if (t == 2 * p.stages + 2) mbar_init(part_go, (uint32_t)S);
     else if (t == 2 * p.stages) mbar_init(tmem_full, (uint32_t)p.nacc);  // one commit per issuing warp
     else if (!p.bulk_push) mbar_init(part_full, kEpiThreads);  // S source CTAs x (4 / S) warps x 32 lanes
     else {
@@ -407,6 +415,11 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
     // ---- this warp's quarter of the partial accumulator -> its owner's shared memory ----
     const bool ok = mbar_wait(tmem_full, 0, p.status, 3);
     tc_fence_after();
+    if (p.part_in_ring) {
+      // the partial tiles that are about to arrive lie where the other CTAs' MMAs have been reading
+      if (ew == 0 && lane < S) mbar_arrive_remote(map_to_cta(part_go, (uint32_t)lane));
+      mbar_wait_cluster(part_go, 0, p.status, 6);
+    }
     const unsigned mask = (p.acc_mask >> (2 * krank)) & 3u;
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
     float* stage = s_stage + (size_t)ew * 32 * (kChunk + 4);
@@ -510,15 +523,34 @@ int launch_router(const void* x, const void* w, int tokens, int d, int experts, 
   p.splitk = p.kblocks >= 16 ? 4 : (p.kblocks >= 4 ? 2 : 1);
   p.num_tiles = ws.num_tiles;
   const int stage_bytes = kBlockTokens * kBlockK * 2 + epad * kBlockK * 2;
-  int fixed = 128 * (epad + 4) * 4 + 4 * epad * 4 + (2 * kMaxStages + 2) * 8 + 16;
+  const int partial_bytes = 128 * (epad + 4) * 4;
   const int transpose_bytes = kEpiWarps * 32 * (kChunk + 4) * 4;
-  int stages = (kSmemLimit - 1024 - fixed) / stage_bytes;
-  if (stages > kMaxStages) stages = kMaxStages;
+  int fixed = 4 * epad * 4 + (2 * kMaxStages + 3) * 8 + 16;
   const int max_fills = (p.kblocks + p.splitk - 1) / p.splitk;
-  if (stages > max_fills) stages = max_fills;
+  const int most = max_fills < kMaxStages ? max_fills : kMaxStages;
+  const auto fit = [&](int behind) { const int n = (kSmemLimit - 1024 - fixed - behind) / stage_bytes; return n < most ? n : most; };
+  int stages = fit(partial_bytes);
+  // The partial tiles take 67 KB at E = 128 and 133 KB at E = 256, behind a ring of 4 and 1 stages.  They may lie
+  // in the ring instead, at the price of one more hand-shake in the cluster (device time, 2049 x 2048, E 256:
+  // 18.0 -> 14.7 us; 8192 x 2048, E 256: 38.7 -> 31.6; 2048 x 4096, E 128: 12.3 -> 11.6; with six stages, E 96,
+  // it was slower: 16387 x 4096: 45.4 -> 47.6).
+  // Which k blocks share an accumulator follows from the stage count and decides the last bits of a logit: a ring
+  // of one stage has one accumulator, an even one two that take turns, and neither changes with the depth.
+  const bool one_acc = stages == 1;
+  p.part_in_ring = 0;
+  if (epad > kChunk && (stages == 1 || stages == 2 || stages == 4) && kSmemLimit - 1024 - fixed >= partial_bytes + transpose_bytes) {
+    const int deeper = one_acc ? fit(0) : fit(0) & ~1;
+    if (deeper > stages) {
+      p.part_in_ring = 1;
+      stages = deeper;
+    }
+  }
+  if (!p.part_in_ring) fixed += partial_bytes;
   if (stages < 1) return fail(MOE_ERR_UNSUPPORTED, "router GEMM: shared memory budget exceeded for experts=%d", experts);
   p.stages = stages;
-  p.stage_in_ring = stages * stage_bytes >= transpose_bytes;
+  p.ring_bytes = stages * stage_bytes;
+  if (p.part_in_ring && p.ring_bytes < partial_bytes + transpose_bytes) p.ring_bytes = partial_bytes + transpose_bytes;
+  p.stage_in_ring = p.part_in_ring || p.ring_bytes >= transpose_bytes;
   {
     static const int bulk_on = [] { const char* v = getenv("MOE_B200_ROUTER_BULK"); return (v && v[0] == '0') ? 0 : 1; }();
     p.bulk_push = (bulk_on && epad == kChunk) ? 1 : 0;
@@ -527,7 +559,7 @@ int launch_router(const void* x, const void* w, int tokens, int d, int experts, 
   }
   if (!p.stage_in_ring) fixed += transpose_bytes;  // few small stages (tiny d_model): the tiles get room of their own
   // every issuing warp needs a stage of its own; both accumulators must fit the 512 TMEM columns
-  p.nacc = kMmaWarps;
+  p.nacc = one_acc ? 1 : kMmaWarps;
   while (p.nacc > 1 && (p.nacc > stages || p.nacc * epad > 512)) p.nacc /= 2;
   int cols = 32;
   while (cols < p.nacc * epad) cols *= 2;
@@ -541,7 +573,7 @@ int launch_router(const void* x, const void* w, int tokens, int d, int experts, 
   }
   p.idx = idx; p.gates = gates; p.logits_out = logits_out;
   p.tile_hist = ws.tile_hist; p.status = ws.status;
-  const size_t smem = 1024 + (size_t)stages * stage_bytes + fixed;
+  const size_t smem = 1024 + (size_t)p.ring_bytes + fixed;
   const int kmax = top_k <= 1 ? 1 : (top_k <= 2 ? 2 : (top_k <= 4 ? 4 : 8));
   auto kernel = kmax == 1 ? router_gemm_select_kernel<1>
                 : kmax == 2 ? router_gemm_select_kernel<2>
