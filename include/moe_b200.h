@@ -17,7 +17,7 @@
  *   - environment switches, read once per process, all default to the fast
  *     path: MOE_B200_PDL=0 (no programmatic dependent launch; moe_set_pdl
  *     changes it at run time); MOE_B200_CTA2_ISSUERS=1 (one MMA-issuing
- *     thread in the grouped GEMM, also moe_set_gemm_mode);
+ *     warp in the grouped GEMM, also moe_set_gemm_mode);
  *     MOE_B200_ROUTER_BULK=0 (router kernel: split-K partials exchanged
  *     with remote stores also where a bulk copy would do),
  *     MOE_B200_ROUTER_PREFETCH=0 (no L2 prefetch of the tokens ahead of the
@@ -92,7 +92,7 @@ int moe_set_pdl(int enabled);
  * Measurement and test helper; no counterpart in the reference. */
 enum {
   MOE_GEMM_TWO_CTA = 1,       /* no effect: every call runs on the two-CTA kernel (tcgen05 cta_group::2) */
-  MOE_GEMM_TWO_ISSUERS = 2,   /* two MMA-issuing threads */
+  MOE_GEMM_TWO_ISSUERS = 2,   /* two MMA-issuing warps */
   MOE_GEMM_TILE_PAIRS = 4,    /* no effect (a variant of a former one-CTA kernel), as the two below */
   MOE_GEMM_M64 = 8,
   MOE_GEMM_TWO_PRODUCERS = 16,

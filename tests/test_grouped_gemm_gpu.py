@@ -348,3 +348,18 @@ def test_grouped_gemm_feature_major_edges(ops, counts, K, N, layout, act, dtype,
     eps = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
     scale = float(ref.abs().max())
     assert ((got - ref).abs() <= 1.5 * eps * ref.abs() + 2e-5 * scale).all()
+
+
+@pytest.mark.parametrize("act", [None, "swiglu"])
+@pytest.mark.parametrize("counts", [[257, 0, 263, 288], [289, 512, 513], [545, 1, 1030]])
+def test_grouped_gemm_units_of_uneven_width(ops, counts, act):
+    """Experts whose 32-row steps do not divide evenly among their units."""
+    off = _segments(counts)
+    g = torch.Generator().manual_seed(sum(counts))
+    n = 128
+    a = torch.randn(off[-1], 192, generator=g).half()
+    w = (torch.randn(len(counts), n * (2 if act == "swiglu" else 1), 192, generator=g) / 14).half()
+    c = ops.grouped_gemm(a.cuda(), w.cuda(), torch.from_numpy(off).cuda(), layout="nk", activation=act)
+    ref = _ref(a, w, off, "nk", act)
+    # one rounding of the result to fp16 (2^-11) on top of fp32 sums of 192 products
+    np.testing.assert_allclose(c.float().cpu().numpy(), ref, rtol=2.0 ** -9, atol=2.0 ** -10)
