@@ -8,8 +8,9 @@
 //
 // Work split: one cluster of SPLITK CTAs per block of 128 tokens; CTA r of the cluster multiplies
 // its slice of the K dimension (d / SPLITK) on the tensor core (UMMA 128 x E x 16, fp32 accumulators
-// in TMEM).  The kernel is bound by the stream of x from HBM, and two per-thread costs would keep it
-// from reaching that bound if one thread did each job:
+// in TMEM); with more blocks a CTA takes several of the slices, whose sums stay apart as long as before.
+// The kernel is bound by the stream of x from HBM, and two per-thread costs would keep it from reaching
+// that bound if one thread did each job:
 //   * the bulk tensor copies of ONE thread are served one after another (about 0.35 us each on
 //     B200 whatever their size): four producer warps issue, each owning every fourth pipeline stage;
 //   * a k block is four short MMAs (E = 64 columns: 32 tensor cycles of work each) and a commit: two warps
@@ -30,7 +31,7 @@
 // 32*(w%4)...), then select.
 #include <cstdlib>
 
-#include "sm100.cuh"
+#include "pack_core.cuh"
 
 namespace moe {
 namespace {
@@ -49,6 +50,11 @@ constexpr int kSelThreads = 32 * (kProducers + kEpiWarps);  // threads that run 
 constexpr int kMaxStages = 12;
 constexpr int kChunk = 64;         // columns moved per transpose step of the partial exchange
 constexpr int kSmemLimit = 227 * 1024;
+constexpr int kSms = 148;
+
+// What a launch does besides one K slice per CTA (kernels of their own: the plain form was 0.5 us slower with the
+// code of the other two in it).
+enum Form { kPlain, kSlices, kPack };  // several slices per CTA; the pack of a small batch
 
 struct RouterParams {
   int tokens, d, experts, top_k;
@@ -59,18 +65,28 @@ struct RouterParams {
   int kblocks, splitk, stages, tmem_cols, num_tiles;
   int ring_bytes;     // pipeline stages (and what reuses them)
   int stage_in_ring;  // the exchange's transpose tiles reuse the pipeline stages
+  int part_bytes;     // partial tiles of the rows that a CTA owns
   int part_in_ring;   // so do the partial tiles, once every CTA of the cluster has finished its MMAs
   int bulk_push;      // the exchange moves a warp's 32 x (E + 4) quarter with one bulk copy (E == 64 only)
   int prefetch_x;     // request this CTA's token boxes into L2 before the dependency wait
-  int nacc;  // MMA-issuing warps = TMEM accumulators (1 or 2; at most the stage count)
-  // bit (2 * k-slice rank + m): issuing warp m gets at least one k-block of that k slice, i.e.
-  // accumulator m holds a partial sum (the other was never written)
+  // K is summed in `slices` slices of at most `nacc` accumulators each, whatever the batch size, so that a
+  // logit's last bits do not depend on how many tokens come with it.  A CTA multiplies `vslices` of them:
+  // k block i of a slice goes to the slice's accumulator (i % period) % nacc.
+  int slices, vslices, period;
+  int nacc;     // accumulators per slice (1 or 2)
+  int issuers;  // MMA-issuing warps (vslices == 1: one per accumulator; else 1)
+  int sources;  // partial tiles per owned row: CTA 0 adds its slices up before it sends them
+  // bit (2 * slice + a): accumulator a of that slice gets at least one k block (the other is never written)
   uint32_t acc_mask;
   int32_t* idx;
   float* gates;
   float* logits_out;
   int32_t* tile_hist;
   int32_t* status;
+  // the pack of a small batch by the same launch (packed == nullptr: not here)
+  const uint4* x;
+  uint4* packed;
+  int32_t *counts, *offsets, *row_route, *route_row;
 };
 
 // A logit that has been rounded to fp16 and its column pack into one 32-bit key whose unsigned
@@ -145,12 +161,17 @@ __device__ __forceinline__ void st_cluster_v4u(uint32_t addr, uint32_t a, uint32
                : "memory");
 }
 
+// First k block of a slice (kblocks * slice / slices, slices = 1, 2 or 4).
+__device__ __forceinline__ int slice_begin(const RouterParams& p, int slice) {
+  return (int)(((unsigned)p.kblocks * (unsigned)slice) >> (p.slices == 4 ? 2 : (p.slices == 2 ? 1 : 0)));
+}
+
 // Select for the rows this CTA owns: kSelThreads threads split every owned row between
 // TPR = kSelThreads / rows threads (consecutive lanes of a warp), each summing the S split-K partials
 // of its 4-column chunks in a fixed order, rounding, biasing and keeping the best KMAX keys; the TPR
 // lists of a row are merged with warp shuffles and lane 0 of the row's group writes the result.
-// Partials of quarter slot s, source CTA c, row r: s_part[((s * S + c) * 32 + r) * EP + column].
-template <int KMAX, int S>
+// Partials of quarter slot s, source tile c, row r: s_part[((s * SRC + c) * 32 + r) * EP + column].
+template <int KMAX, int S, int SRC>
 __device__ __forceinline__ void select_rows(const RouterParams& p, const float* __restrict__ s_part,
                                             int32_t* __restrict__ s_hist, int st, int block, int krank) {
   constexpr int ROWS = kBlockTokens / S;   // rows this CTA owns
@@ -161,7 +182,7 @@ __device__ __forceinline__ void select_rows(const RouterParams& p, const float* 
   const int slot = ro >> 5, r = ro & 31;
   const int q = slot * S + krank;  // TMEM lane quarter == 32-token group of the block
   const int row = block * kBlockTokens + q * 32 + r;
-  const float* prow = s_part + (size_t)((slot * S) * 32 + r) * EP;
+  const float* prow = s_part + (size_t)((slot * SRC) * 32 + r) * EP;
   float* lrow = (p.logits_out != nullptr && row < p.tokens) ? p.logits_out + (size_t)row * EL : nullptr;
 
   uint32_t keys[KMAX];
@@ -171,7 +192,7 @@ __device__ __forceinline__ void select_rows(const RouterParams& p, const float* 
     const int c0 = ch * 4;
     float4 a = *reinterpret_cast<const float4*>(prow + c0);
 #pragma unroll
-    for (int src = 1; src < S; ++src) {
+    for (int src = 1; src < SRC; ++src) {
       const float4 b = *reinterpret_cast<const float4*>(prow + (size_t)src * 32 * EP + c0);
       a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
     }
@@ -216,7 +237,7 @@ __device__ __forceinline__ void select_rows(const RouterParams& p, const float* 
 // After the exchange: wait until all partials of the rows this CTA owns have arrived, select, and
 // write the histogram of every 32-token group the CTA owns.  Run by the kSelThreads threads of the
 // producer and epilogue warps (st = index among them).
-template <int KMAX>
+template <int KMAX, Form FORM>
 __device__ __forceinline__ void select_phase(const RouterParams& p, const float* s_partial, int32_t* s_hist,
                                              uint32_t part_full, int st, int block, int krank) {
   const int S = p.splitk;
@@ -227,9 +248,14 @@ __device__ __forceinline__ void select_phase(const RouterParams& p, const float*
     cluster_arrive_relaxed();
   }
   if (__all_sync(0xffffffffu, arrived)) {  // warp-uniform: select_rows shuffles
-    if (S == 4) select_rows<KMAX, 4>(p, s_partial, s_hist, st, block, krank);
-    else if (S == 2) select_rows<KMAX, 2>(p, s_partial, s_hist, st, block, krank);
-    else select_rows<KMAX, 1>(p, s_partial, s_hist, st, block, krank);
+    if constexpr (FORM == kSlices) {
+      if (S == 2) select_rows<KMAX, 2, 3>(p, s_partial, s_hist, st, block, krank);
+      else select_rows<KMAX, 1, 1>(p, s_partial, s_hist, st, block, krank);
+    } else {
+      if (S == 4) select_rows<KMAX, 4, 4>(p, s_partial, s_hist, st, block, krank);
+      else if (S == 2) select_rows<KMAX, 2, 2>(p, s_partial, s_hist, st, block, krank);
+      else select_rows<KMAX, 1, 1>(p, s_partial, s_hist, st, block, krank);
+    }
   }
   asm volatile("bar.sync 1, 256;" ::: "memory");  // the kSelThreads threads only
   if (p.tile_hist != nullptr) {
@@ -242,7 +268,52 @@ __device__ __forceinline__ void select_phase(const RouterParams& p, const float*
   }
 }
 
-template <int KMAX>
+// The pack of a small batch (at most kTileTokens tokens, kPackRoutes routes, kPackItems pieces of 2 KB per warp)
+// by the one cluster that has routed it: every CTA ranks the tile (its indices and histogram come from CTA 0, which owns
+// those rows) and copies its share of the pieces, whose loads are under way while it ranks.  One launch instead
+// of two: a route of 16 x 4096, E 64, k 2 takes a caller 19.4 instead of 22.0 us (the device 11.4 either way).
+constexpr int kPackPiece = 128;  // 16-byte vectors
+constexpr int kPackItems = 2;
+constexpr int kPackRoutes = 64;  // 32 x 2048, E 256, k 8 (256 rows to store): 22.5 us in two launches, 25.0 in one
+inline int pack_pieces(int d) { return (d / 8 + kPackPiece - 1) / kPackPiece; }
+
+__device__ __forceinline__ void pack_small(const RouterParams& p, uint8_t* smem, int krank) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // (the MMA warps have not waited yet)
+  const int n_vec = p.d / 8;
+  const int pieces = (n_vec + kPackPiece - 1) / kPackPiece;
+  const int lane = threadIdx.x & 31;
+  uint4 r[kPackItems][kPackPiece / 32];
+  int tok[kPackItems], v0[kPackItems];
+#pragma unroll
+  for (int i = 0; i < kPackItems; ++i) {
+    const int item = (i * p.splitk + krank) * (kThreads / 32) + (threadIdx.x >> 5);
+    tok[i] = item / pieces;
+    v0[i] = (item - tok[i] * pieces) * kPackPiece + lane;
+#pragma unroll
+    for (int u = 0; u < kPackPiece / 32; ++u)
+      if (tok[i] < p.tokens && v0[i] + u * 32 < n_vec) r[i][u] = __ldg(p.x + (size_t)tok[i] * n_vec + v0[i] + u * 32);
+  }
+  cluster_sync_all();  // CTA 0's indices and histogram are visible, every ring is free
+  int32_t* s_base = reinterpret_cast<int32_t*>(smem);
+  int32_t* s_total = s_base + p.experts;
+  int32_t* s_dst = s_total + p.experts;
+  tile_destinations(p.idx, p.tile_hist, nullptr, p.counts, p.offsets, p.row_route, p.route_row, 0, 0,
+                    p.tokens * p.top_k, p.experts, p.top_k, 1, krank == 0, krank == 0, s_base, s_total, s_dst,
+                    p.status);
+#pragma unroll
+  for (int i = 0; i < kPackItems; ++i) {
+    if (tok[i] >= p.tokens) break;
+    for (int j = 0; j < p.top_k; ++j) {
+      const int row = s_dst[tok[i] * p.top_k + j];
+      if (row < 0) continue;
+#pragma unroll
+      for (int u = 0; u < kPackPiece / 32; ++u)
+        if (v0[i] + u * 32 < n_vec) p.packed[(size_t)row * n_vec + v0[i] + u * 32] = r[i][u];
+    }
+  }
+}
+
+template <int KMAX, Form FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
                           const __grid_constant__ CUtensorMap tmap_w, const RouterParams p) {
@@ -261,13 +332,13 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
   const int EP = E + 4;  // padded row of a partial tile: conflict-free 128-bit accesses
   uint8_t* sA = smem;
   uint8_t* sB = sA + (size_t)p.stages * kABytes;
-  // partial tiles [4][32][EP] behind the ring, or at its start; transpose tiles of the exchange [4 warps][32]
-  // [kChunk + 4]: the ring itself once the last MMA has read it (the usual case; behind the partial tiles where
-  // those are in the ring too), else a region of their own
+  // partial tiles [4 / S][sources][32][EP] behind the ring, or at its start; transpose tiles of the exchange
+  // [4 warps][32][kChunk + 4]: the ring itself once the last MMA has read it (the usual case; behind the partial
+  // tiles where those are in the ring too), else a region of their own
   float* s_tail = reinterpret_cast<float*>(smem + p.ring_bytes);
   float* s_partial = p.part_in_ring ? reinterpret_cast<float*>(smem) : s_tail;
-  if (!p.part_in_ring) s_tail += (size_t)4 * 32 * EP;
-  float* s_stage = p.part_in_ring ? s_partial + (size_t)4 * 32 * EP
+  if (!p.part_in_ring) s_tail += p.part_bytes / 4;
+  float* s_stage = p.part_in_ring ? s_partial + p.part_bytes / 4
                                   : (p.stage_in_ring ? reinterpret_cast<float*>(smem) : s_tail);
   if (!p.stage_in_ring) s_tail += kEpiWarps * 32 * (kChunk + 4);
   int32_t* s_hist = reinterpret_cast<int32_t*>(s_tail);  // [4][E]
@@ -279,6 +350,7 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
   const int block = blockIdx.x;
   const int krank = (int)cluster_ctarank();
   const int S = p.splitk;
+  const int vslices = FORM == kSlices ? p.vslices : 1;
   // this CTA's k blocks: kblocks * krank / S with S = 1, 2 or 4 (shifts: the prologue is on the
   // critical path of the first copy)
   const int sh = S == 4 ? 2 : (S == 2 ? 1 : 0);
@@ -310,7 +382,7 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
     if (t < p.stages) mbar_init(full0 + 8 * t, 1);
     else if (t < 2 * p.stages) mbar_init(empty0 + 8 * (t - p.stages), 1);
     else if (t == 2 * p.stages + 2) mbar_init(part_go, (uint32_t)S);
-    else if (t == 2 * p.stages) mbar_init(tmem_full, (uint32_t)p.nacc);  // one commit per issuing warp
+    else if (t == 2 * p.stages) mbar_init(tmem_full, (uint32_t)p.issuers);  // one commit per issuing warp
     else if (!p.bulk_push) mbar_init(part_full, kEpiThreads);  // S source CTAs x (4 / S) warps x 32 lanes
     else {
       // bulk exchange: the four quarters this CTA owns arrive as byte counts on the barrier
@@ -359,7 +431,7 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
     }
     __syncwarp();
     cluster_wait_acquire();
-    select_phase<KMAX>(p, s_partial, s_hist, part_full, warp * 32 + lane, block, krank);
+    select_phase<KMAX, FORM>(p, s_partial, s_hist, part_full, warp * 32 + lane, block, krank);
   } else if (warp < kProducers + kMmaWarps) {
     // ------------------------------ MMA issuers (the first also owns the TMEM allocation) ---------------
     // Issuing warp m owns the stages s with s % nacc == m, consumes their fills in order and
@@ -373,27 +445,39 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
     asm volatile("bar.sync 2, 192;" ::: "memory");  // MMA + epilogue warps: the TMEM address is published
     tc_fence_after();
     const uint32_t tmem_base = *s_tmem;
-    if (m < p.nacc) {  // the whole warp; an elected lane issues
+    if (m < p.issuers) {  // the whole warp; an elected lane issues
       const uint32_t idesc = make_idesc_f16(kBlockTokens, E, p.bf16, 0, 0);
-      bool fresh = true;  // accumulator m holds nothing yet
+      uint32_t written = 0;  // accumulators that hold something
       int s_next = 0, owner = 0;
       uint32_t ph_next = 0;
+      int v = 0, turn = 0, slice_end = FORM == kSlices ? slice_begin(p, krank * vslices + 1) - kb0 : 0;
       for (int it = 0; it < nkb; ++it) {
         const int s = s_next, owner_now = owner;
         const uint32_t ph = ph_next;
-        if (++owner == p.nacc) owner = 0;
+        if (++owner == p.issuers) owner = 0;
         if (++s_next == p.stages) { s_next = 0; owner = 0; ph_next ^= 1u; }
+        int acc = m;  // one slice per CTA: the issuing warp's own accumulator
+        if constexpr (FORM == kSlices) {
+          if (it == slice_end) {
+            ++v;
+            turn = 0;
+            slice_end = slice_begin(p, krank * vslices + v + 1) - kb0;
+          }
+          acc = v * p.nacc + (p.nacc == 2 ? (turn & 1) : 0);
+          if (++turn == p.period) turn = 0;
+        }
         if (owner_now != m) continue;
         if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph, p.status, 2))) break;
         tc_fence_after();
         const uint64_t adesc = make_desc_kmajor_sw128(smem_u32(sA + (size_t)s * kABytes));
         const uint64_t bdesc = make_desc_kmajor_sw128(smem_u32(sB + (size_t)s * b_bytes));
+        const uint32_t more = FORM == kSlices ? (written >> acc) & 1u : written;
 #pragma unroll
         for (int k = 0; k < kBlockK / kUmmaK; ++k) {
           // +32 bytes per K step inside the 128-byte swizzle row (address field is in 16-byte units)
-          umma_f16(tmem_base + (uint32_t)(m * E), adesc + 2 * k, bdesc + 2 * k, idesc, (uint32_t)(!fresh || k != 0));
+          umma_f16(tmem_base + (uint32_t)(acc * E), adesc + 2 * k, bdesc + 2 * k, idesc, k != 0 ? 1u : more);
         }
-        fresh = false;
+        written = FORM == kSlices ? written | 1u << acc : 1u;
         umma_commit(empty0 + 8 * s);  // stage may be refilled once these MMAs have read it
       }
       umma_commit(tmem_full);  // this warp's accumulator is complete (or abandoned: the epilogue must not hang)
@@ -420,74 +504,90 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
       if (ew == 0 && lane < S) mbar_arrive_remote(map_to_cta(part_go, (uint32_t)lane));
       mbar_wait_cluster(part_go, 0, p.status, 6);
     }
-    const unsigned mask = (p.acc_mask >> (2 * krank)) & 3u;
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
     float* stage = s_stage + (size_t)ew * 32 * (kChunk + 4);
-    // row (slot * S + krank) * 32 + r of the owner's partial buffer
-    const uint32_t owner_part = map_to_cta(smem_u32(s_partial), (uint32_t)dest) + (uint32_t)((slot * S + krank) * 32 * EP) * 4u;
-    for (int c0 = 0; c0 < E; c0 += kChunk) {
-      const int width = min(kChunk, E - c0);  // 16, 32, 48 or 64 columns
-      // (1) sum the accumulators of this chunk: thread = row, registers = columns; the loads of 32 columns are
-      // in flight together.  (2) transpose through this warp's staging tile so that a store instruction covers
-      // whole rows.
-      __syncwarp();  // the previous chunk has been read out of the staging tile
+    // CTA 0 sends the sum of its slices (the first ones of the fixed order), the others every slice for itself
+    const int tiles = FORM == kSlices && krank != 0 ? vslices : 1;
+    for (int tile = 0; tile < tiles; ++tile) {
+      const int v0 = FORM == kSlices && krank != 0 ? tile : 0;
+      const int v1 = FORM == kSlices && krank == 0 ? vslices : v0 + 1;
+      // source tile `at` of the rows of this quarter in the owner's partial buffer
+      const int at = FORM == kSlices && krank != 0 ? 1 + (krank - 1) * vslices + tile : krank;
+      const int sources = FORM == kSlices ? p.sources : S;
+      const uint32_t owner_part =
+          map_to_cta(smem_u32(s_partial), (uint32_t)dest) + (uint32_t)((slot * sources + at) * 32 * EP) * 4u;
+      for (int c0 = 0; c0 < E; c0 += kChunk) {
+        const int width = min(kChunk, E - c0);  // 16, 32, 48 or 64 columns
+        // (1) sum the accumulators of this chunk: thread = row, registers = columns; the loads of 32 columns are
+        // in flight together.  (2) transpose through this warp's staging tile so that a store instruction covers
+        // whole rows.
+        __syncwarp();  // the previous chunk has been read out of the staging tile
 #pragma unroll
-      for (int h = 0; h < kChunk; h += 32) {
-        uint32_t r[kMmaWarps][32];
+        for (int h = 0; h < kChunk; h += 32) {
+          float sum[32];
+          const auto add_slice = [&](int v, bool first) {
+            const unsigned mask = (p.acc_mask >> (2 * (krank * vslices + v))) & 3u;
+            uint32_t r[kMmaWarps][32];
 #pragma unroll
-        for (int a = 0; a < kMmaWarps; ++a)
+            for (int a = 0; a < kMmaWarps; ++a)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) r[a][i] = 0u;
-        if (ok && h < width) {
+              for (int i = 0; i < 32; ++i) r[a][i] = 0u;
+            if (ok && h < width) {
 #pragma unroll
-          for (int a = 0; a < kMmaWarps; ++a) {
-            if (a < p.nacc && ((mask >> a) & 1u)) {
+              for (int a = 0; a < kMmaWarps; ++a) {
+                if (a < p.nacc && ((mask >> a) & 1u)) {
 #pragma unroll
-              for (int g = 0; g < 2; ++g)
-                if (h + g * 16 < width)
-                  tmem_ld16_nowait(taddr + (uint32_t)(a * E + c0 + h + g * 16), reinterpret_cast<uint32_t(&)[16]>(r[a][g * 16]));
+                  for (int g = 0; g < 2; ++g)
+                    if (h + g * 16 < width)
+                      tmem_ld16_nowait(taddr + (uint32_t)((v * p.nacc + a) * E + c0 + h + g * 16),
+                                       reinterpret_cast<uint32_t(&)[16]>(r[a][g * 16]));
+                }
+              }
+              tmem_ld_wait();
             }
-          }
-          tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              float part = __uint_as_float(r[0][i]);
+#pragma unroll
+              for (int a = 1; a < kMmaWarps; ++a) part += __uint_as_float(r[a][i]);
+              sum[i] = first ? part : sum[i] + part;
+            }
+          };
+          add_slice(v0, true);
+          if constexpr (FORM == kSlices)
+            for (int v = v0 + 1; v < v1; ++v) add_slice(v, false);
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(stage + lane * (kChunk + 4) + h + i) =
+                make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
         }
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          float v[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            v[u] = __uint_as_float(r[0][i + u]);
-#pragma unroll
-            for (int a = 1; a < kMmaWarps; ++a) v[u] += __uint_as_float(r[a][i + u]);
-          }
-          *reinterpret_cast<float4*>(stage + lane * (kChunk + 4) + h + i) = make_float4(v[0], v[1], v[2], v[3]);
-        }
-      }
-      __syncwarp();
-      if (p.bulk_push) {
-        // (3a) E == 64: the staging tile has the layout of the owner's block (32 rows of E + 4 floats),
-        // so one bulk copy moves the quarter and counts its bytes on the owner's barrier: no remote
-        // store instructions and no release-arrive behind them
-        fence_proxy_async();  // this lane's staging writes, for the async proxy
         __syncwarp();
-        if (lane == 0)
-          bulk_copy_to_cluster(owner_part, smem_u32(stage), (uint32_t)(32 * (kChunk + 4) * sizeof(float)),
-                               map_to_cta(part_full, (uint32_t)dest));
-        break;
-      }
-      // (3) 16 lanes x 16 bytes cover the (up to) 64 columns of one row: two rows per instruction
-      const int cl = (lane & 15) * 4;
-      if (cl < width) {
-#pragma unroll 4
-        for (int r2 = 0; r2 < 32; r2 += 2) {
-          const int r = r2 + (lane >> 4);
-          const float4 t = *reinterpret_cast<const float4*>(stage + r * (kChunk + 4) + cl);
-          st_cluster_v4u(owner_part + (uint32_t)(r * EP + c0 + cl) * 4u, __float_as_uint(t.x), __float_as_uint(t.y),
-                         __float_as_uint(t.z), __float_as_uint(t.w));
+        if (p.bulk_push) {
+          // (3a) E == 64: the staging tile has the layout of the owner's block (32 rows of E + 4 floats),
+          // so one bulk copy moves the quarter and counts its bytes on the owner's barrier: no remote
+          // store instructions and no release-arrive behind them
+          fence_proxy_async();  // this lane's staging writes, for the async proxy
+          __syncwarp();
+          if (lane == 0)
+            bulk_copy_to_cluster(owner_part, smem_u32(stage), (uint32_t)(32 * (kChunk + 4) * sizeof(float)),
+                                 map_to_cta(part_full, (uint32_t)dest));
+          break;
+        }
+        // (3) 16 lanes x 16 bytes cover the (up to) 64 columns of one row: two rows per instruction
+        const int cl = (lane & 15) * 4;
+        if (cl < width) {
+  #pragma unroll 4
+          for (int r2 = 0; r2 < 32; r2 += 2) {
+            const int r = r2 + (lane >> 4);
+            const float4 t = *reinterpret_cast<const float4*>(stage + r * (kChunk + 4) + cl);
+            st_cluster_v4u(owner_part + (uint32_t)(r * EP + c0 + cl) * 4u, __float_as_uint(t.x), __float_as_uint(t.y),
+                           __float_as_uint(t.z), __float_as_uint(t.w));
+          }
         }
       }
     }
     if (!p.bulk_push) mbar_arrive_remote(map_to_cta(part_full, (uint32_t)dest));  // releases this thread's stores
-    select_phase<KMAX>(p, s_partial, s_hist, part_full, (kProducers + ew) * 32 + lane, block, krank);
+    select_phase<KMAX, FORM>(p, s_partial, s_hist, part_full, (kProducers + ew) * 32 + lane, block, krank);
   }
 
   tc_fence_before();
@@ -501,11 +601,32 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
   // MMA warps on their way here), so when it completes every copy of the cluster has landed and no
   // CTA's shared memory is still being read.
   if (p.bulk_push) cluster_wait_acquire();
+  if constexpr (FORM == kPack) pack_small(p, smem, krank);
 }
+
+using RouterKernel = void (*)(const CUtensorMap, const CUtensorMap, const RouterParams);
+template <Form FORM>
+RouterKernel router_kernel(int kmax) {
+  return kmax == 1   ? router_gemm_select_kernel<1, FORM>
+         : kmax == 2 ? router_gemm_select_kernel<2, FORM>
+         : kmax == 4 ? router_gemm_select_kernel<4, FORM>
+                     : router_gemm_select_kernel<8, FORM>;
+}
+
+int k_slices(int d) {
+  const int kblocks = (d + kBlockK - 1) / kBlockK;
+  return kblocks >= 16 ? 4 : (kblocks >= 4 ? 2 : 1);
+}
+
+// Where the router kernel packs the rows itself.
+struct PackOut {
+  void* packed;
+  int32_t *counts, *offsets, *row_route, *route_row;
+};
 
 int launch_router(const void* x, const void* w, int tokens, int d, int experts, int top_k, int skew_experts,
                   float skew_bias, int dtype, int32_t* idx, float* gates, float* logits_out, const Workspace& ws,
-                  cudaStream_t stream) {
+                  cudaStream_t stream, const PackOut* pack = nullptr) {
   const int epad = (experts + 15) / 16 * 16;  // W rows past `experts` are zero-filled by the TMA unit
   CUtensorMap tmap_x, tmap_w;
   int rc = encode_tmap_2d(&tmap_x, x, (uint64_t)tokens, (uint64_t)d, (uint64_t)d * 2, kBlockK, kBlockTokens);
@@ -520,65 +641,92 @@ int launch_router(const void* x, const void* w, int tokens, int d, int experts, 
   p.skew_bias = skew_bias;
   if (skew_bias == 0.0f) p.skew_experts = 0;
   p.kblocks = (d + kBlockK - 1) / kBlockK;
-  p.splitk = p.kblocks >= 16 ? 4 : (p.kblocks >= 4 ? 2 : 1);
+  p.slices = k_slices(d);
   p.num_tiles = ws.num_tiles;
   const int stage_bytes = kBlockTokens * kBlockK * 2 + epad * kBlockK * 2;
-  const int partial_bytes = 128 * (epad + 4) * 4;
   const int transpose_bytes = kEpiWarps * 32 * (kChunk + 4) * 4;
   int fixed = 4 * epad * 4 + (2 * kMaxStages + 3) * 8 + 16;
-  const int max_fills = (p.kblocks + p.splitk - 1) / p.splitk;
-  const int most = max_fills < kMaxStages ? max_fills : kMaxStages;
-  const auto fit = [&](int behind) { const int n = (kSmemLimit - 1024 - fixed - behind) / stage_bytes; return n < most ? n : most; };
-  int stages = fit(partial_bytes);
+  const auto fit = [&](int behind, int slices_per_cta) {
+    const int fills = (p.kblocks * slices_per_cta + p.slices - 1) / p.slices;
+    const int most = fills < kMaxStages ? fills : kMaxStages;
+    const int n = (kSmemLimit - 1024 - fixed - behind) / stage_bytes;
+    return n < most ? n : most;
+  };
+  // One slice per CTA and its partial tiles behind the ring: what decides which k blocks share an accumulator.
+  const int slice_part = 128 * (epad + 4) * 4;
+  p.period = fit(slice_part, 1);
+  p.nacc = kMmaWarps;
+  while (p.nacc > 1 && (p.nacc > p.period || p.nacc * epad > 512)) p.nacc /= 2;
+  // A second wave of CTAs costs a whole start-up, exchange and select: with more CTAs than SMs a CTA takes two
+  // slices, or all four, as far as their accumulators fit TMEM and three stages fit beside the partial tiles.
+  // Same sums in the same order (device time, one slice per CTA -> this rule: 4800 x 1024, E 64: 11.9 -> 9.0 us;
+  // 8192 x 2048, E 32: 14.2 -> 12.1; 16387 x 4096, E 64: 41.0 -> 30.9).
+  const int blocks = (tokens + kBlockTokens - 1) / kBlockTokens;
+  const auto part_of = [&](int v) {
+    const int ctas = p.slices / v, sources = 1 + (ctas - 1) * v;
+    return 4 / ctas * sources * 32 * (epad + 4) * 4;
+  };
+  p.vslices = 1;
+  while (p.vslices < p.slices && blocks * (p.slices / p.vslices) > kSms && 2 * p.vslices * p.nacc * epad <= 512 &&
+         fit(part_of(2 * p.vslices), 2 * p.vslices) >= 3)
+    p.vslices *= 2;
+  p.splitk = p.slices / p.vslices;
+  p.sources = 1 + (p.splitk - 1) * p.vslices;
+  p.part_bytes = part_of(p.vslices);
+  int stages = fit(p.part_bytes, p.vslices);
   // The partial tiles take 67 KB at E = 128 and 133 KB at E = 256, behind a ring of 4 and 1 stages.  They may lie
   // in the ring instead, at the price of one more hand-shake in the cluster (device time, 2049 x 2048, E 256:
-  // 18.0 -> 14.7 us; 8192 x 2048, E 256: 38.7 -> 31.6; 2048 x 4096, E 128: 12.3 -> 11.6; with six stages, E 96,
-  // it was slower: 16387 x 4096: 45.4 -> 47.6).
-  // Which k blocks share an accumulator follows from the stage count and decides the last bits of a logit: a ring
-  // of one stage has one accumulator, an even one two that take turns, and neither changes with the depth.
-  const bool one_acc = stages == 1;
+  // 18.0 -> 14.4 us; 8192 x 2048, E 256: 38.7 -> 31.6; 2048 x 4096, E 128: 12.3 -> 11.6; with six stages, E 96,
+  // it was slower: 16387 x 4096: 45.4 -> 47.6).  With two issuing warps the depth stays even: they own every
+  // second stage, and which of them has a k block must not change.
   p.part_in_ring = 0;
-  if (epad > kChunk && (stages == 1 || stages == 2 || stages == 4) && kSmemLimit - 1024 - fixed >= partial_bytes + transpose_bytes) {
-    const int deeper = one_acc ? fit(0) : fit(0) & ~1;
+  if (epad > kChunk && stages <= 4 && (p.vslices > 1 || stages != 3) &&
+      kSmemLimit - 1024 - fixed >= p.part_bytes + transpose_bytes) {
+    const int deeper = p.nacc == 1 || p.vslices > 1 ? fit(0, p.vslices) : fit(0, p.vslices) & ~1;
     if (deeper > stages) {
       p.part_in_ring = 1;
       stages = deeper;
     }
   }
-  if (!p.part_in_ring) fixed += partial_bytes;
+  if (!p.part_in_ring) fixed += p.part_bytes;
   if (stages < 1) return fail(MOE_ERR_UNSUPPORTED, "router GEMM: shared memory budget exceeded for experts=%d", experts);
   p.stages = stages;
   p.ring_bytes = stages * stage_bytes;
-  if (p.part_in_ring && p.ring_bytes < partial_bytes + transpose_bytes) p.ring_bytes = partial_bytes + transpose_bytes;
+  if (p.part_in_ring && p.ring_bytes < p.part_bytes + transpose_bytes) p.ring_bytes = p.part_bytes + transpose_bytes;
   p.stage_in_ring = p.part_in_ring || p.ring_bytes >= transpose_bytes;
   {
     static const int bulk_on = [] { const char* v = getenv("MOE_B200_ROUTER_BULK"); return (v && v[0] == '0') ? 0 : 1; }();
-    p.bulk_push = (bulk_on && epad == kChunk) ? 1 : 0;
+    p.bulk_push = (bulk_on && epad == kChunk && p.vslices == 1) ? 1 : 0;
     static const int pf_on = [] { const char* v = getenv("MOE_B200_ROUTER_PREFETCH"); return (v && v[0] == '0') ? 0 : 1; }();
     p.prefetch_x = pf_on;
   }
   if (!p.stage_in_ring) fixed += transpose_bytes;  // few small stages (tiny d_model): the tiles get room of their own
-  // every issuing warp needs a stage of its own; both accumulators must fit the 512 TMEM columns
-  p.nacc = one_acc ? 1 : kMmaWarps;
-  while (p.nacc > 1 && (p.nacc > stages || p.nacc * epad > 512)) p.nacc /= 2;
+  // every issuing warp needs a stage of its own
+  p.issuers = p.vslices == 1 ? p.nacc : 1;
   int cols = 32;
-  while (cols < p.nacc * epad) cols *= 2;
+  while (cols < p.vslices * p.nacc * epad) cols *= 2;
   p.tmem_cols = cols;
   p.acc_mask = 0;
-  for (int r = 0; r < p.splitk; ++r) {
-    const int k0 = (int)(((long long)p.kblocks * r) / p.splitk), k1 = (int)(((long long)p.kblocks * (r + 1)) / p.splitk);
+  for (int r = 0; r < p.slices; ++r) {
+    const int k0 = (int)(((long long)p.kblocks * r) / p.slices), k1 = (int)(((long long)p.kblocks * (r + 1)) / p.slices);
     unsigned mask = 0;
-    for (int it = 0; it < k1 - k0; ++it) mask |= 1u << ((it % stages) % p.nacc);
+    for (int it = 0; it < k1 - k0; ++it) mask |= 1u << ((it % p.period) % p.nacc);
     p.acc_mask |= mask << (2 * r);
   }
   p.idx = idx; p.gates = gates; p.logits_out = logits_out;
   p.tile_hist = ws.tile_hist; p.status = ws.status;
+  p.x = static_cast<const uint4*>(x);
+  p.packed = nullptr;
+  if (pack != nullptr) {
+    p.packed = static_cast<uint4*>(pack->packed);
+    p.counts = pack->counts; p.offsets = pack->offsets; p.row_route = pack->row_route; p.route_row = pack->route_row;
+  }
   const size_t smem = 1024 + (size_t)p.ring_bytes + fixed;
   const int kmax = top_k <= 1 ? 1 : (top_k <= 2 ? 2 : (top_k <= 4 ? 4 : 8));
-  auto kernel = kmax == 1 ? router_gemm_select_kernel<1>
-                : kmax == 2 ? router_gemm_select_kernel<2>
-                : kmax == 4 ? router_gemm_select_kernel<4>
-                            : router_gemm_select_kernel<8>;
+  const int form = pack != nullptr ? kPack : (p.vslices > 1 ? kSlices : kPlain);
+  auto kernel = form == kPack     ? router_kernel<kPack>(kmax)
+                : form == kSlices ? router_kernel<kSlices>(kmax)
+                                  : router_kernel<kPlain>(kmax);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((tokens + kBlockTokens - 1) / kBlockTokens, p.splitk, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
@@ -595,8 +743,8 @@ int launch_router(const void* x, const void* w, int tokens, int d, int experts, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  static SmemGrant grants[4];  // one per KMAX
-  cudaError_t e = grant_smem(reinterpret_cast<const void*>(kernel), smem, grants[kmax == 8 ? 3 : kmax >> 1]);
+  static SmemGrant grants[3][4];  // one per form and KMAX
+  cudaError_t e = grant_smem(reinterpret_cast<const void*>(kernel), smem, grants[form][kmax == 8 ? 3 : kmax >> 1]);
   if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "router GEMM: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   e = cudaLaunchKernelEx(&cfg, kernel, tmap_x, tmap_w, p);
   if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "router_gemm_select_kernel: %s", cudaGetErrorString(e));
@@ -653,9 +801,14 @@ extern "C" int moe_route_fused(const void* x, const void* w_router, int dtype, i
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Workspace ws = carve(workspace, tokens, experts);
   if (tokens > 0) {
+    // one launch for a small batch (the router has already required 16-byte rows and alignment of x)
+    const PackOut out = {packed, counts, offsets, row_route, route_row};
+    const bool one = tokens <= kTileTokens && tokens * top_k <= kPackRoutes &&
+                     tokens * pack_pieces(d) <= kPackItems * k_slices(d) * (kThreads / 32) && packed != nullptr &&
+                     (reinterpret_cast<uintptr_t>(packed) & 15) == 0;
     rc = launch_router(x, w_router, tokens, d, experts, top_k, skew_experts, skew_bias, dtype, idx, gates, logits_out,
-                       ws, s);
-    if (rc != MOE_OK) return rc;
+                       ws, s, one ? &out : nullptr);
+    if (rc != MOE_OK || one) return rc;
   }
   return launch_scan_scatter(x, 2, idx, tokens, d, experts, top_k, counts, offsets, packed, row_route, route_row,
                              ws, s);
