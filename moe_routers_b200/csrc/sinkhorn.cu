@@ -250,9 +250,10 @@ sinkhorn_kernel(const SParams p) {
 //                 mbarrier, so that no CTA waits for a cluster-wide barrier
 // with two block-wide barriers and one mbarrier wait.  Every sum is added in an order that depends on the
 // shape alone and is the same in every CTA.
-// T = 4096, E = 64, 10 iterations: 44.0 -> 23.2 us on the device (the shared-memory form below held K in
-// shared memory, one thread per row, and exchanged partials behind a cluster barrier); 256 x 64: 12.9 us,
-// 8192 x 32: 20.9 us.  Larger matrices keep the forms below (16384 x 64: 76 us).
+// T = 4096, E = 64, 10 iterations: 44.0 -> 21.3 us on the device (the shared-memory form below: K in shared
+// memory, one thread per row, partials exchanged behind a cluster barrier), of which 1.3 per iteration, 1.0 per
+// pick and the rest launch, loads and exponentials; 256 x 64: 12.7 us, 8192 x 32: 19.1, 8192 x 64: 36.9.  Larger
+// matrices keep the forms below (16384 x 64: 76 us).
 constexpr int kRegThreads = 512;
 constexpr int kRegWarps = kRegThreads / 32;
 constexpr int kRegCols = 8;    // columns per lane
@@ -308,25 +309,36 @@ __device__ __forceinline__ void st_async_v4(uint32_t dst_cluster, const float (&
                : "memory");
 }
 
-// 8 consecutive logits of a row as fp32 (columns past E: not touched).
-template <typename T>
-__device__ __forceinline__ void load_logits8(const SParams& p, int row, int c0, float (&v)[kRegCols]) {
-  const T* src = static_cast<const T*>(p.logits) + (size_t)row * p.experts + c0;
+// 8 consecutive logits of RPL rows (RG rows apart) as fp32; rows and columns past the end: -inf.  All loads are
+// under way before the first is used: one round trip to memory, not one per row.
+template <typename T, int RPL, int RG>
+__device__ __forceinline__ void load_logits(const SParams& p, int row0, int c0, float (&k)[RPL][kRegCols]) {
+  const T* src = static_cast<const T*>(p.logits) + (size_t)row0 * p.experts + c0;
+  const size_t step = (size_t)RG * p.experts;
   if (p.vec_rows && c0 + kRegCols <= p.experts) {
-    constexpr int W = 16 / sizeof(T);
-    union { uint4 q[kRegCols / W]; T e[kRegCols]; } u;
+    constexpr int W = 16 / sizeof(T), Q = kRegCols / W;
+    union Piece { uint4 q[Q]; T e[kRegCols]; } u[RPL];
 #pragma unroll
-    for (int i = 0; i < kRegCols / W; ++i) u.q[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+    for (int r = 0; r < RPL; ++r)
 #pragma unroll
-    for (int j = 0; j < kRegCols; ++j) v[j] = to_float(u.e[j]);
+      for (int i = 0; i < Q; ++i)
+        if (row0 + r * RG < p.tokens) u[r].q[i] = __ldg(reinterpret_cast<const uint4*>(src + r * step) + i);
+#pragma unroll
+    for (int r = 0; r < RPL; ++r)
+#pragma unroll
+      for (int j = 0; j < kRegCols; ++j) k[r][j] = row0 + r * RG < p.tokens ? to_float(u[r].e[j]) : -INFINITY;
   } else {
 #pragma unroll
-    for (int j = 0; j < kRegCols; ++j)
-      if (c0 + j < p.experts) v[j] = to_float(src[j]);
+    for (int r = 0; r < RPL; ++r)
+#pragma unroll
+      for (int j = 0; j < kRegCols; ++j)
+        k[r][j] = row0 + r * RG < p.tokens && c0 + j < p.experts ? to_float(src[r * step + j]) : -INFINITY;
   }
   if (p.temperature != 1.0f) {
 #pragma unroll
-    for (int j = 0; j < kRegCols; ++j) v[j] = to_float(from_float<T>(v[j] / p.temperature));
+    for (int r = 0; r < RPL; ++r)
+#pragma unroll
+      for (int j = 0; j < kRegCols; ++j) k[r][j] = to_float(from_float<T>(k[r][j] / p.temperature));
   }
 }
 
@@ -363,17 +375,9 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
   const int rg = lane / LPR, c0 = (lane % LPR) * kRegCols;
   const int row0 = (int)blockIdx.x * p.rows_per_cta + warp * (RG * RPL) + rg;  // + r * RG
   float k[RPL][kRegCols];
-#pragma unroll
-  for (int r = 0; r < RPL; ++r) {
-    const int row = row0 + r * RG;
-#pragma unroll
-    for (int j = 0; j < kRegCols; ++j) k[r][j] = -INFINITY;
-    if (row < p.tokens && c0 < E) {
-      if (p.logits_dtype == MOE_F16) load_logits8<__half>(p, row, c0, k[r]);
-      else if (p.logits_dtype == MOE_BF16) load_logits8<__nv_bfloat16>(p, row, c0, k[r]);
-      else load_logits8<float>(p, row, c0, k[r]);
-    }
-  }
+  if (p.logits_dtype == MOE_F16) load_logits<__half, RPL, RG>(p, row0, c0, k);
+  else if (p.logits_dtype == MOE_BF16) load_logits<__nv_bfloat16, RPL, RG>(p, row0, c0, k);
+  else load_logits<float, RPL, RG>(p, row0, c0, k);
 #pragma unroll
   for (int r = 0; r < RPL; ++r) {
     float m = k[r][0];
@@ -381,9 +385,9 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
     for (int j = 1; j < kRegCols; ++j) m = fmaxf(m, k[r][j]);
 #pragma unroll
     for (int ofs = 1; ofs < LPR; ofs <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, ofs));
-    const bool in_row = row0 + r * RG < p.tokens;
+    if (row0 + r * RG >= p.tokens) m = 0.f;
 #pragma unroll
-    for (int j = 0; j < kRegCols; ++j) k[r][j] = in_row && c0 + j < E ? expf(k[r][j] - m) : 0.f;
+    for (int j = 0; j < kRegCols; ++j) k[r][j] = expf(k[r][j] - m);  // past the matrix: -inf -> 0
   }
 
   // the row scales this lane is responsible for (1 inside the matrix, 0 past its end)
@@ -485,12 +489,8 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
 #pragma unroll
   for (int r = 0; r < RPL; ++r) {
     const int row = row0 + r * RG;
-    uint32_t taken = 0;
 #pragma unroll
-    for (int j = 0; j < kRegCols; ++j) {
-      k[r][j] = a[r] * k[r][j] * b[j];
-      if (c0 + j >= E) taken |= 1u << j;
-    }
+    for (int j = 0; j < kRegCols; ++j) k[r][j] = c0 + j < E ? a[r] * k[r][j] * b[j] : -INFINITY;
     float sum = 0.f;
     float pv[8];
     int pi[8];
@@ -500,16 +500,17 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
         float bv = -INFINITY;
         int bi = 0x7fffffff;
 #pragma unroll
-        for (int j = 0; j < kRegCols; ++j)
-          if (!((taken >> j) & 1u) && better(k[r][j], c0 + j, bv, bi)) { bv = k[r][j]; bi = c0 + j; }
+        for (int j = 0; j < kRegCols; ++j)  // ascending columns: the first of equal values stays
+          if (k[r][j] > bv) { bv = k[r][j]; bi = c0 + j; }
 #pragma unroll
         for (int ofs = 1; ofs < LPR; ofs <<= 1) {
           const float ov = __shfl_xor_sync(0xffffffffu, bv, ofs);
           const int oi = __shfl_xor_sync(0xffffffffu, bi, ofs);
           if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
         }
-        const int local = bi - c0;
-        if ((unsigned)local < (unsigned)kRegCols) taken |= 1u << local;
+#pragma unroll
+        for (int j = 0; j < kRegCols; ++j)
+          if (bi == c0 + j) k[r][j] = -INFINITY;  // taken (q itself is never negative)
         pv[t] = bv;
         pi[t] = bi;
         sum += bv;
