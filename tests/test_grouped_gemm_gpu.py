@@ -308,6 +308,40 @@ def test_grouped_gemm_sm_margin_same_result(ops):
         assert torch.equal(got.view(torch.int16), ref.view(torch.int16)), margin
 
 
+@pytest.mark.parametrize("experts,per_expert,K,N,margin", [
+    (8, 4096, 4096, 4096, 32),    # two long calls that leave 32 SMs free
+    (1, 256, 98304, 12800, 0),    # 50 work units each: the other SMs are free
+])
+def test_consecutive_grouped_gemms_leave_room_for_another_stream(ops, experts, per_expert, K, N, margin):
+    """Two calls in a row run one after the other: the second one's CTAs must not sit on the SMs that the first
+    one leaves free, where nothing else fits beside their shared memory.  An independent kernel on another stream,
+    enqueued while the first call runs, is then through at once; with the second call waiting on those SMs it has
+    to wait until the first one leaves its own, half-way through the two."""
+    import time
+
+    a = torch.randn(experts * per_expert, K, device="cuda").half()
+    w = (torch.randn(experts, N, K, device="cuda", dtype=torch.float16) / K ** 0.5)
+    off = torch.arange(0, experts * per_expert + 1, per_expert, dtype=torch.int32, device="cuda")
+    out = torch.empty(experts * per_expert, N, dtype=torch.float16, device="cuda")
+    side, other = torch.cuda.Stream(), torch.zeros(4096, device="cuda")
+    shares = []
+    for _ in range(6):
+        start, done, beside = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+        torch.cuda.synchronize()
+        start.record()
+        for _ in range(2):
+            ops.grouped_gemm(a, w, off, layout="nk", out=out, sm_margin=margin)
+        done.record()
+        time.sleep(5e-5)
+        with torch.cuda.stream(side):
+            other.add_(1)
+            beside.record()
+        torch.cuda.synchronize()
+        shares.append(start.elapsed_time(beside) / start.elapsed_time(done))
+    assert ops.read_status() == 0
+    assert sorted(shares[1:])[2] < 0.4, shares
+
+
 @pytest.mark.parametrize("counts,K,N,layout,act,dtype", [
     ([1], 8, 16, "nk", None, torch.float16),                            # the smallest call
     ([31, 32, 33, 0, 255, 256, 257], 136, 272, "nk", "gelu", torch.float16),   # unit edges; a feature tile of 16
