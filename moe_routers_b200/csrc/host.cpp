@@ -10,6 +10,7 @@
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <ATen/ATen.h>
 
@@ -18,6 +19,19 @@
 
 namespace {
 
+// The GIL is given up for as long as one of these lives: an allocation may have to wait for the device, whose
+// work may in turn need a launch by another Python thread.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
+struct TensorSpec {
+  at::ScalarType type;
+  int64_t sizes[3];
+  int dims;
+};
+
 PyObject* empties(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 2 && PyTuple_Check(args[1]), "empties(device_index, ((dtype, size, ..), ..))");
@@ -25,30 +39,33 @@ PyObject* empties(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (dev == -1 && PyErr_Occurred()) return nullptr;
   const at::TensorOptions on_gpu = at::TensorOptions().device(at::Device(at::kCUDA, (c10::DeviceIndex)dev));
   const Py_ssize_t count = PyTuple_GET_SIZE(args[1]);
-  PyObject* out = PyTuple_New(count);
-  if (out == nullptr) return nullptr;
-  try {
-    for (Py_ssize_t i = 0; i < count; ++i) {
-      PyObject* spec = PyTuple_GET_ITEM(args[1], i);
-      TORCH_CHECK(PyTuple_Check(spec) && PyTuple_GET_SIZE(spec) >= 1 && PyTuple_GET_SIZE(spec) <= 4 &&
-                      THPDtype_Check(PyTuple_GET_ITEM(spec, 0)),
-                  "empties: (dtype, up to three sizes) expected");
-      int64_t sizes[3];
-      const Py_ssize_t dims = PyTuple_GET_SIZE(spec) - 1;
-      for (Py_ssize_t d = 0; d < dims; ++d) {
-        sizes[d] = PyLong_AsLongLong(PyTuple_GET_ITEM(spec, d + 1));
-        if (sizes[d] == -1 && PyErr_Occurred()) throw python_error();
-      }
-      const at::ScalarType type = reinterpret_cast<THPDtype*>(PyTuple_GET_ITEM(spec, 0))->scalar_type;
-      PyObject* t = THPVariable_Wrap(at::empty(at::IntArrayRef(sizes, dims), on_gpu.dtype(type)));
-      if (t == nullptr) throw python_error();
-      PyTuple_SET_ITEM(out, i, t);
+  c10::SmallVector<TensorSpec, 8> specs(count);
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    PyObject* spec = PyTuple_GET_ITEM(args[1], i);
+    TORCH_CHECK(PyTuple_Check(spec) && PyTuple_GET_SIZE(spec) >= 1 && PyTuple_GET_SIZE(spec) <= 4 &&
+                    THPDtype_Check(PyTuple_GET_ITEM(spec, 0)),
+                "empties: (dtype, up to three sizes) expected");
+    specs[i].type = reinterpret_cast<THPDtype*>(PyTuple_GET_ITEM(spec, 0))->scalar_type;
+    specs[i].dims = (int)PyTuple_GET_SIZE(spec) - 1;
+    for (int d = 0; d < specs[i].dims; ++d) {
+      specs[i].sizes[d] = PyLong_AsLongLong(PyTuple_GET_ITEM(spec, d + 1));
+      if (specs[i].sizes[d] == -1 && PyErr_Occurred()) return nullptr;
     }
-  } catch (...) {
-    Py_DECREF(out);
-    throw;
   }
-  return out;
+  c10::SmallVector<at::Tensor, 8> tensors(count);
+  {
+    WithoutGil released;
+    for (Py_ssize_t i = 0; i < count; ++i)
+      tensors[i] = at::empty(at::IntArrayRef(specs[i].sizes, specs[i].dims), on_gpu.dtype(specs[i].type));
+  }
+  THPObjectPtr out(PyTuple_New(count));
+  if (!out) return nullptr;
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    PyObject* t = THPVariable_Wrap(std::move(tensors[i]));
+    if (t == nullptr) return nullptr;
+    PyTuple_SET_ITEM(out.get(), i, t);
+  }
+  return out.release();
   END_HANDLE_TH_ERRORS
 }
 

@@ -48,6 +48,40 @@ def test_empties_are_plain_tensors():
 
 
 @pytest.mark.gpu
+def test_empties_let_other_threads_run():
+    """An allocation may wait for the device; a thread that has to launch the work it waits for must not be kept
+    out meanwhile.  Many tensors in one call: nearly all of its time is the allocator's, and another thread's
+    longest standstill stays well below it."""
+    import threading
+    import time
+
+    from moe_routers_b200._host import empties
+
+    specs = ((torch.uint8, 1),) * 200_000
+    torch.empty(1, device="cuda")
+    gaps, stop, running = [], threading.Event(), threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+            running.set()
+
+    t = threading.Thread(target=tick)
+    t.start()
+    running.wait()
+    begin = time.perf_counter()
+    out = empties(0, specs)
+    took = time.perf_counter() - begin
+    stop.set()
+    t.join()
+    assert len(out) == len(specs)
+    assert max(gaps) < 0.6 * took, (max(gaps), took)
+
+
+@pytest.mark.gpu
 def test_layer_sees_changed_weights():
     layer = _layer(8).half().cuda().requires_grad_(False)
     x = torch.randn(1, 16, 64, device="cuda").half()
