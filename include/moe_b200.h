@@ -86,17 +86,16 @@ long long moe_launch_count(void);
  * after the call.  Measurement helper; no counterpart in the reference. */
 int moe_set_pdl(int enabled);
 
-/* Variants of the grouped GEMM: one or two MMA-issuing warps (MOE_GEMM_TWO_ISSUERS), the same result
- * bits either way; the default (two) is the faster one.  moe_set_gemm_mode(mode) replaces the set for
- * launches issued after the call (process-wide) and returns the previous one; a negative mode only
- * reads it.  Measurement and test helper; no counterpart in the reference.  The other bits are
- * reserved: they chose among kernels that are gone, and are accepted and kept without effect. */
+/* Variants the grouped GEMM may use; every combination computes the same result bits, the default
+ * (all on) is the fastest measured.  moe_set_gemm_mode(mode) replaces the set for launches issued
+ * after the call (process-wide) and returns the previous one; a negative mode only reads it.
+ * Measurement and test helper; no counterpart in the reference. */
 enum {
-  MOE_GEMM_TWO_CTA = 1,       /* reserved */
-  MOE_GEMM_TWO_ISSUERS = 2,
-  MOE_GEMM_TILE_PAIRS = 4,    /* reserved */
-  MOE_GEMM_M64 = 8,           /* reserved */
-  MOE_GEMM_TWO_PRODUCERS = 16,/* reserved */
+  MOE_GEMM_TWO_CTA = 1,       /* no effect: every call runs on the two-CTA kernel (tcgen05 cta_group::2) */
+  MOE_GEMM_TWO_ISSUERS = 2,   /* two MMA-issuing warps */
+  MOE_GEMM_TILE_PAIRS = 4,    /* no effect (a variant of a former one-CTA kernel), as the two below */
+  MOE_GEMM_M64 = 8,
+  MOE_GEMM_TWO_PRODUCERS = 16,
   MOE_GEMM_ALL = 31
 };
 int moe_set_gemm_mode(int mode);
@@ -241,8 +240,7 @@ int moe_router_gemm_select(const void* x, const void* w_router, int dtype, int t
  *   idx [tokens, top_k] int32, gates [tokens, top_k] float32.
  * Limits: top_k <= 8, experts <= 1024, tokens * experts * 4 bytes / (number of SMs) must fit in
  * shared memory (about 7 M matrix entries on a B200).  Up to 524288 entries (experts <= 256, rounded up to
- * 8 * 2^n) stay in the registers of one thread-block cluster, up to about 800 k in its shared memory (16 CTAs;
- * half as many entries where the cluster has 8); larger ones run as a cooperative grid
+ * 8 * 2^n) stay in the registers of one thread-block cluster; larger ones run as a cooperative grid
  * with one grid barrier per iteration; if a barrier wait gives up, the status block records it
  * and the workspace must be re-initialised with moe_workspace_init.
  */

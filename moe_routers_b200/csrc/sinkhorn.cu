@@ -15,7 +15,6 @@
 // run-to-run deterministic).  One grid barrier per iteration; the grid is launched cooperatively so
 // that all CTAs are co-resident, and the barrier spin is bounded in time.
 #include <atomic>
-#include <cfloat>
 #include <cstdlib>
 
 #include "sm100.cuh"
@@ -51,14 +50,6 @@ __device__ __forceinline__ void store_pick(const SParams& p, size_t at, int pick
   if (p.gate_dtype == MOE_F32) static_cast<float*>(p.gates)[at] = gate;
   else if (p.gate_dtype == MOE_F16) static_cast<__half*>(p.gates)[at] = __float2half_rn(gate);
   else static_cast<__nv_bfloat16*>(p.gates)[at] = __float2bfloat16_rn(gate);
-}
-
-// The column step: b_j <- b_j * (T/E) / (b_j * sum_i a_i K_ij + eps).  Where a column is empty (an expert whose
-// logits are all -inf or far below the others) b_j grows by T/E / eps in every iteration; it is kept finite, so
-// that q = a * 0 * b stays 0, as it does where q itself is iterated.  (NaN passes.)
-__device__ __forceinline__ float next_column_scale(float b, float sum, float eps, float ct) {
-  const float next = b / (b * sum + eps) * ct;
-  return next > FLT_MAX ? FLT_MAX : next;
 }
 
 // One thread per row: scan q_ij = a_i K_ij b_j over the columns keeping the best KMAX entries under
@@ -193,7 +184,7 @@ sinkhorn_kernel(const SParams p) {
         float s = 0.f;
         for (int c = 0; c < nblk; ++c) s += all[(size_t)c * E + j];  // same order in every CTA
         const float b = s_b[j];
-        s_b[j] = next_column_scale(b, s, p.eps, ct);
+        s_b[j] = b / (b * s + p.eps) * ct;
       }
       __syncthreads();
     } else {
@@ -231,7 +222,7 @@ sinkhorn_kernel(const SParams p) {
         float s = 0.f;
         for (int gg = 0; gg < groups; ++gg) s += s_part[(size_t)gg * E + j];
         const float b = s_b[j];
-        s_b[j] = next_column_scale(b, s, p.eps, ct);
+        s_b[j] = b / (b * s + p.eps) * ct;
       }
       __syncthreads();
     }
@@ -418,10 +409,7 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
     if ((i * 2 * kRegWarps + 2 * warp + half) * 4 + col_in_quad < E) b_own[i] = 1.f;
   const float ct = (float)p.tokens / (float)max(E, 1);
 
-  // The exchange that this thread has given up because its wait ran into the limit.  It then takes no further part
-  // in any: it stores nothing, so that the CTAs that count on its sums give up in their turn, and arms nothing (a
-  // phase that has not completed must not be armed again).  The kernel runs to its end; the status block says why.
-  int given_up = p.iters;
+  bool ok = true;
   for (int it = 0;; ++it) {
     // ---- row step: a_i <- a_i / (a_i * sum_j K_ij b_j + eps) ----
     float b[kRegCols];
@@ -471,15 +459,14 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
         float v[4] = {t.x, t.y, t.z, t.w};
         reduce_lanes<4, 1, 16>(v, src);
         spread_lanes<4, 1, 16>(v, src);
-        if (src < nblk && given_up == p.iters)
+        if (src < nblk)
           st_async_v4(sm100::map_to_cta(sm100::smem_u32(all + me * SP + quad * 4), (uint32_t)src), v,
                       sm100::map_to_cta(bar, (uint32_t)src));
       }
     }
-    if (given_up == p.iters) {
-      if (!sm100::mbar_wait_cluster(bar, (uint32_t)(it >> 1) & 1u, p.status, 9)) given_up = it;
-      else if (threadIdx.x == 0) sm100::mbar_expect_tx(bar, tx_bytes);  // the buffer's next use, two iterations on
-    }
+    // (a wait that gives up is not repeated: the kernel runs to its end and the status block says why)
+    if (ok) ok = sm100::mbar_wait_cluster(bar, (uint32_t)(it >> 1) & 1u, p.status, 9);
+    if (threadIdx.x == 0) sm100::mbar_expect_tx(bar, tx_bytes);  // the buffer's next use, two iterations on
 #pragma unroll
     for (int i = 0; i < QPH; ++i) {
       const int quad = i * 2 * kRegWarps + 2 * warp + half;
@@ -488,7 +475,7 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
         if (src < nblk) t = *reinterpret_cast<const float4*>(all + src * SP + quad * 4);
         float v[4] = {t.x, t.y, t.z, t.w};
         reduce_lanes<4, 1, 16>(v, src);
-        b_own[i] = next_column_scale(b_own[i], v[0], p.eps, ct);
+        b_own[i] = b_own[i] / (b_own[i] * v[0] + p.eps) * ct;
         if (src < 4) s_b[quad * 4 + col_in_quad] = b_own[i];
       }
     }
@@ -538,10 +525,6 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
   }
   // no CTA leaves while another may still store into its shared memory
   sm100::cluster_sync_all();
-  // Nobody stores any more, but what was stored for an exchange that was given up, and for the one behind it (no
-  // CTA gets past that), may still be under way to this CTA: one more limited wait for each.
-  for (int late = given_up; late < min(given_up + 2, p.iters); ++late)
-    (void)sm100::mbar_wait_cluster(bar0 + 8u * (uint32_t)(late & 1), (uint32_t)(late >> 1) & 1u, p.status, 9);
 }
 
 using RegKernel = void (*)(const SParams);
@@ -579,22 +562,15 @@ bool places_wide_cluster(RegKernel kernel, const cudaLaunchConfig_t& cfg) {
   return v == 2;
 }
 
-// MOE_B200_SINKHORN_CLUSTER=8 in the environment keeps every cluster at the portable size.
-bool wide_clusters_allowed() {
-  static const bool allowed = [] { const char* v = getenv("MOE_B200_SINKHORN_CLUSTER"); return !(v && atoi(v) == 8); }();
-  return allowed;
-}
-
 // Launches the register kernel where the matrix fits one cluster's registers: at most 64 elements a thread,
-// 16 CTAs (8 where the device cannot place 16 or the environment keeps the portable size), E <= 256:
-// T * E <= 524288 (262144) with E rounded up to 8 * 2^n.
+// 16 CTAs (8 where the device cannot place 16), E <= 256: T * E <= 524288 with E rounded up to 8 * 2^n.
 // MOE_ERR_UNSUPPORTED, with nothing launched, where it does not.
 int launch_sinkhorn_regs(SParams p, cudaStream_t s) {
   int lpr = 1;
   while (lpr * kRegCols < p.experts) lpr *= 2;
   if (lpr > 32) return MOE_ERR_UNSUPPORTED;
   const int rows_per_set = kRegWarps * (32 / lpr);  // rows per CTA and row slot of a lane
-  for (int max_ctas = wide_clusters_allowed() ? kRegMaxCtas : kRegMaxCtas / 2; max_ctas >= kRegMaxCtas / 2; max_ctas /= 2) {
+  for (int max_ctas = kRegMaxCtas; max_ctas >= kRegMaxCtas / 2; max_ctas /= 2) {
     int rpl = 1;
     while (rpl <= 8 && (long long)rows_per_set * rpl * max_ctas < p.tokens) rpl *= 2;
     if (rpl > 8) return MOE_ERR_UNSUPPORTED;
@@ -738,9 +714,11 @@ int sinkhorn_route(const void* logits, int logits_dtype, int tokens, int experts
 
   // One cluster when the matrix fits its shared memory (T=4096, E=64 does): no global round trips
   // inside the iterations.  16 CTAs where the device can place such a cluster (half the rows per CTA:
-  // every pass of the iteration is shorter), else the portable 8.
+  // every pass of the iteration is shorter), else the portable 8.  MOE_B200_SINKHORN_CLUSTER=8 in the
+  // environment keeps the portable size.
+  static const int wide_ok = [] { const char* v = getenv("MOE_B200_SINKHORN_CLUSTER"); return !(v && atoi(v) == 8); }();
   for (int ctas : {kClusterCtasWide, kClusterCtas}) {
-    if (ctas == kClusterCtasWide && (!wide_clusters_allowed() || tokens < 1024)) continue;
+    if (ctas == kClusterCtasWide && (!wide_ok || tokens < 1024)) continue;
     const int rows = (tokens + ctas - 1) / ctas;
     const size_t smem = sinkhorn_smem(rows, experts, kClusterThreads, ctas, true);
     if (smem <= 200 * 1024 && tokens >= 256) {
