@@ -240,7 +240,8 @@ int moe_router_gemm_select(const void* x, const void* w_router, int dtype, int t
  *   idx [tokens, top_k] int32, gates [tokens, top_k] float32.
  * Limits: top_k <= 8, experts <= 1024, tokens * experts * 4 bytes / (number of SMs) must fit in
  * shared memory (about 7 M matrix entries on a B200).  Up to 524288 entries (experts <= 256, rounded up to
- * 8 * 2^n) stay in the registers of one thread-block cluster; larger ones run as a cooperative grid
+ * 8 * 2^n) stay in the registers of one thread-block cluster, up to about 800 k in its shared memory (16 CTAs;
+ * half as many entries where the cluster has 8); larger ones run as a cooperative grid
  * with one grid barrier per iteration; if a barrier wait gives up, the status block records it
  * and the workspace must be re-initialised with moe_workspace_init.
  */

@@ -562,15 +562,22 @@ bool places_wide_cluster(RegKernel kernel, const cudaLaunchConfig_t& cfg) {
   return v == 2;
 }
 
+// MOE_B200_SINKHORN_CLUSTER=8 in the environment keeps every cluster at the portable size.
+bool wide_clusters_allowed() {
+  static const bool allowed = [] { const char* v = getenv("MOE_B200_SINKHORN_CLUSTER"); return !(v && atoi(v) == 8); }();
+  return allowed;
+}
+
 // Launches the register kernel where the matrix fits one cluster's registers: at most 64 elements a thread,
-// 16 CTAs (8 where the device cannot place 16), E <= 256: T * E <= 524288 with E rounded up to 8 * 2^n.
+// 16 CTAs (8 where the device cannot place 16 or the environment keeps the portable size), E <= 256:
+// T * E <= 524288 (262144) with E rounded up to 8 * 2^n.
 // MOE_ERR_UNSUPPORTED, with nothing launched, where it does not.
 int launch_sinkhorn_regs(SParams p, cudaStream_t s) {
   int lpr = 1;
   while (lpr * kRegCols < p.experts) lpr *= 2;
   if (lpr > 32) return MOE_ERR_UNSUPPORTED;
   const int rows_per_set = kRegWarps * (32 / lpr);  // rows per CTA and row slot of a lane
-  for (int max_ctas = kRegMaxCtas; max_ctas >= kRegMaxCtas / 2; max_ctas /= 2) {
+  for (int max_ctas = wide_clusters_allowed() ? kRegMaxCtas : kRegMaxCtas / 2; max_ctas >= kRegMaxCtas / 2; max_ctas /= 2) {
     int rpl = 1;
     while (rpl <= 8 && (long long)rows_per_set * rpl * max_ctas < p.tokens) rpl *= 2;
     if (rpl > 8) return MOE_ERR_UNSUPPORTED;
@@ -714,11 +721,9 @@ int sinkhorn_route(const void* logits, int logits_dtype, int tokens, int experts
 
   // One cluster when the matrix fits its shared memory (T=4096, E=64 does): no global round trips
   // inside the iterations.  16 CTAs where the device can place such a cluster (half the rows per CTA:
-  // every pass of the iteration is shorter), else the portable 8.  MOE_B200_SINKHORN_CLUSTER=8 in the
-  // environment keeps the portable size.
-  static const int wide_ok = [] { const char* v = getenv("MOE_B200_SINKHORN_CLUSTER"); return !(v && atoi(v) == 8); }();
+  // every pass of the iteration is shorter), else the portable 8.
   for (int ctas : {kClusterCtasWide, kClusterCtas}) {
-    if (ctas == kClusterCtasWide && (!wide_ok || tokens < 1024)) continue;
+    if (ctas == kClusterCtasWide && (!wide_clusters_allowed() || tokens < 1024)) continue;
     const int rows = (tokens + ctas - 1) / ctas;
     const size_t smem = sinkhorn_smem(rows, experts, kClusterThreads, ctas, true);
     if (smem <= 200 * 1024 && tokens >= 256) {

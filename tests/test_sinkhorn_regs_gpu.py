@@ -1,6 +1,10 @@
 """The Sinkhorn kernel that keeps the matrix in registers, at the edges of its layouts: columns per lane,
 rows per lane, CTAs per cluster, and the shapes just outside of it, against the reference's iteration
 (models/decoder_moe.py:92-123) in 64 bits."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -63,3 +67,43 @@ def test_sinkhorn_unaligned_logits():
     b = a.clone()
     for x, y in zip(ops.sinkhorn(a, 4), ops.sinkhorn(b, 4)):
         assert torch.equal(x, y)
+
+
+def _ctas(t, e):
+    """CTAs of the one kernel that a call launches, read from its captured graph."""
+    from cuda.bindings import driver
+
+    from moe_routers_b200 import ops
+
+    logits = torch.zeros(t, e, device="cuda")
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ops.sinkhorn(logits, 1)  # the stream's workspace exists
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        ops.sinkhorn(logits, 1)
+    handle = driver.CUgraph(graph.raw_cuda_graph())
+    _, _, count = driver.cuGraphGetNodes(handle)
+    _, nodes, _ = driver.cuGraphGetNodes(handle, count)
+    kernels = [n for n in nodes if driver.cuGraphNodeGetType(n)[1] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL]
+    assert len(kernels) == 1
+    err, params = driver.cuGraphKernelNodeGetParams(kernels[0])
+    assert err == driver.CUresult.CUDA_SUCCESS
+    return params.gridDimX
+
+
+def test_sinkhorn_keeps_the_portable_cluster_size_when_told():
+    """MOE_B200_SINKHORN_CLUSTER=8, read once per process: every shape of this file in a process that has it
+    set, and no cluster above 8 CTAs (4096 x 64 and 1024 x 256 fill 8 CTAs' registers)."""
+    env = dict(os.environ, MOE_B200_SINKHORN_CLUSTER="8")
+    here = os.path.abspath(__file__)
+    root = os.path.dirname(os.path.dirname(here))
+    code = (f"import sys; sys.path[:0] = [{root!r}, {os.path.dirname(here)!r}]; import test_sinkhorn_regs_gpu as t; "
+            "print([t._ctas(*s) for s in ((4096, 64), (1024, 256), (600, 64))])")
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, cwd=root)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.strip().endswith("[8, 8, 8]"), r.stdout
+    r = subprocess.run([sys.executable, "-m", "pytest", here, "-q", "-x", "-k", "layout_edges or unaligned",
+                        "-p", "no:cacheprovider"], env=env, capture_output=True, text=True, cwd=root)
+    assert r.returncode == 0, r.stdout[-3000:]
