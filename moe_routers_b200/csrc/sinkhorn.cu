@@ -409,7 +409,10 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
     if ((i * 2 * kRegWarps + 2 * warp + half) * 4 + col_in_quad < E) b_own[i] = 1.f;
   const float ct = (float)p.tokens / (float)max(E, 1);
 
-  bool ok = true;
+  // The exchange that this thread has given up because its wait ran into the limit.  It then takes no further part
+  // in any: it stores nothing, so that the CTAs that count on its sums give up in their turn, and arms nothing (a
+  // phase that has not completed must not be armed again).  The kernel runs to its end; the status block says why.
+  int given_up = p.iters;
   for (int it = 0;; ++it) {
     // ---- row step: a_i <- a_i / (a_i * sum_j K_ij b_j + eps) ----
     float b[kRegCols];
@@ -459,14 +462,15 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
         float v[4] = {t.x, t.y, t.z, t.w};
         reduce_lanes<4, 1, 16>(v, src);
         spread_lanes<4, 1, 16>(v, src);
-        if (src < nblk)
+        if (src < nblk && given_up == p.iters)
           st_async_v4(sm100::map_to_cta(sm100::smem_u32(all + me * SP + quad * 4), (uint32_t)src), v,
                       sm100::map_to_cta(bar, (uint32_t)src));
       }
     }
-    // (a wait that gives up is not repeated: the kernel runs to its end and the status block says why)
-    if (ok) ok = sm100::mbar_wait_cluster(bar, (uint32_t)(it >> 1) & 1u, p.status, 9);
-    if (threadIdx.x == 0) sm100::mbar_expect_tx(bar, tx_bytes);  // the buffer's next use, two iterations on
+    if (given_up == p.iters) {
+      if (!sm100::mbar_wait_cluster(bar, (uint32_t)(it >> 1) & 1u, p.status, 9)) given_up = it;
+      else if (threadIdx.x == 0) sm100::mbar_expect_tx(bar, tx_bytes);  // the buffer's next use, two iterations on
+    }
 #pragma unroll
     for (int i = 0; i < QPH; ++i) {
       const int quad = i * 2 * kRegWarps + 2 * warp + half;
@@ -525,6 +529,10 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
   }
   // no CTA leaves while another may still store into its shared memory
   sm100::cluster_sync_all();
+  // Nobody stores any more, but what was stored for an exchange that was given up, and for the one behind it (no
+  // CTA gets past that), may still be under way to this CTA: one more limited wait for each.
+  for (int late = given_up; late < min(given_up + 2, p.iters); ++late)
+    (void)sm100::mbar_wait_cluster(bar0 + 8u * (uint32_t)(late & 1), (uint32_t)(late >> 1) & 1u, p.status, 9);
 }
 
 using RegKernel = void (*)(const SParams);
