@@ -10,6 +10,7 @@ or driver.
 from __future__ import annotations
 
 import glob
+import importlib.metadata
 import importlib.util
 import os
 import shutil
@@ -23,6 +24,7 @@ LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libmoe_b200.so")
 HOST_SRC = os.path.join(CSRC, "host.cpp")
 HOST_PATH = os.path.join(PKG, "_host.so")
+HOST_STAMP = os.path.join(LIB_DIR, "host_stamp.txt")  # what _host.so was built for
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
 NVCC_FLAGS = [
@@ -52,14 +54,34 @@ def _stale() -> bool:
     return any(os.path.getmtime(p) > t for p in deps)
 
 
+def _host_stamp() -> str:
+    """What _host.so depends on besides its source: it reads torch's and Python's own structures."""
+    return f"torch {importlib.metadata.version('torch')} {sysconfig.get_config_var('SOABI')}\n"
+
+
+def _host_fresh(stamp: str) -> bool:
+    if not os.path.exists(HOST_PATH) or os.path.getmtime(HOST_PATH) < os.path.getmtime(HOST_SRC):
+        return False
+    try:
+        with open(HOST_STAMP) as f:
+            return f.read() == stamp
+    except FileNotFoundError:
+        return False
+
+
 def build_host(force: bool = False) -> str:
-    """Compile csrc/host.cpp against the installed torch's headers into the extension module _host.so."""
-    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= os.path.getmtime(HOST_SRC):
+    """Compile csrc/host.cpp against the installed torch's headers into the extension module _host.so (no-op if it
+    is newer than its source and was built for this torch and this Python)."""
+    stamp = _host_stamp()
+    if not force and _host_fresh(stamp):
         return HOST_PATH
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    import torch
+
+    torch_dir = os.path.dirname(torch.__file__)
     includes = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
                 sysconfig.get_paths()["include"]]
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=1"]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     for path in includes:
         cmd += ["-isystem", path]
     cmd += [HOST_SRC, "-o", HOST_PATH, "-L", os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
@@ -67,12 +89,22 @@ def build_host(force: bool = False) -> str:
     if r.returncode != 0:
         sys.stderr.write(r.stdout)
         raise RuntimeError(f"g++ failed on {HOST_SRC}")
+    os.makedirs(LIB_DIR, exist_ok=True)
+    with open(HOST_STAMP, "w") as f:
+        f.write(stamp)
     return HOST_PATH
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compile every .cu under csrc/ into lib/libmoe_b200.so and host.cpp into _host.so (no-op if fresh)."""
-    build_host(force)
+    """Compile every .cu under csrc/ into lib/libmoe_b200.so, and where torch is installed host.cpp into _host.so
+    (no-op if fresh)."""
+    path = _build_cuda(force, verbose)
+    if importlib.util.find_spec("torch") is not None:
+        build_host(force)
+    return path
+
+
+def _build_cuda(force: bool, verbose: bool) -> str:
     if not force and not _stale():
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)
