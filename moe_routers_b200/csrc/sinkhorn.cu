@@ -15,6 +15,7 @@
 // run-to-run deterministic).  One grid barrier per iteration; the grid is launched cooperatively so
 // that all CTAs are co-resident, and the barrier spin is bounded in time.
 #include <atomic>
+#include <cfloat>
 #include <cstdlib>
 
 #include "sm100.cuh"
@@ -50,6 +51,14 @@ __device__ __forceinline__ void store_pick(const SParams& p, size_t at, int pick
   if (p.gate_dtype == MOE_F32) static_cast<float*>(p.gates)[at] = gate;
   else if (p.gate_dtype == MOE_F16) static_cast<__half*>(p.gates)[at] = __float2half_rn(gate);
   else static_cast<__nv_bfloat16*>(p.gates)[at] = __float2bfloat16_rn(gate);
+}
+
+// The column step: b_j <- b_j * (T/E) / (b_j * sum_i a_i K_ij + eps).  Where a column is empty (an expert whose
+// logits are all -inf or far below the others) b_j grows by T/E / eps in every iteration; it is kept finite, so
+// that q = a * 0 * b stays 0, as it does where q itself is iterated.  (NaN passes.)
+__device__ __forceinline__ float next_column_scale(float b, float sum, float eps, float ct) {
+  const float next = b / (b * sum + eps) * ct;
+  return next > FLT_MAX ? FLT_MAX : next;
 }
 
 // One thread per row: scan q_ij = a_i K_ij b_j over the columns keeping the best KMAX entries under
@@ -184,7 +193,7 @@ sinkhorn_kernel(const SParams p) {
         float s = 0.f;
         for (int c = 0; c < nblk; ++c) s += all[(size_t)c * E + j];  // same order in every CTA
         const float b = s_b[j];
-        s_b[j] = b / (b * s + p.eps) * ct;
+        s_b[j] = next_column_scale(b, s, p.eps, ct);
       }
       __syncthreads();
     } else {
@@ -222,7 +231,7 @@ sinkhorn_kernel(const SParams p) {
         float s = 0.f;
         for (int gg = 0; gg < groups; ++gg) s += s_part[(size_t)gg * E + j];
         const float b = s_b[j];
-        s_b[j] = b / (b * s + p.eps) * ct;
+        s_b[j] = next_column_scale(b, s, p.eps, ct);
       }
       __syncthreads();
     }
@@ -479,7 +488,7 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
         if (src < nblk) t = *reinterpret_cast<const float4*>(all + src * SP + quad * 4);
         float v[4] = {t.x, t.y, t.z, t.w};
         reduce_lanes<4, 1, 16>(v, src);
-        b_own[i] = b_own[i] / (b_own[i] * v[0] + p.eps) * ct;
+        b_own[i] = next_column_scale(b_own[i], v[0], p.eps, ct);
         if (src < 4) s_b[quad * 4 + col_in_quad] = b_own[i];
       }
     }

@@ -58,6 +58,27 @@ def test_sinkhorn_layout_edges(t, e, k, iters, dtype):
     assert torch.equal(ridx, idx.long()) and torch.equal(rw, w.to(dtype))
 
 
+@pytest.mark.parametrize("t,e", [(300, 64), (70, 16), (40, 256), (300, 60), (200, 257), (8193, 64), (16384, 64)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_sinkhorn_masked_columns(t, e, dtype):
+    """Logits of -inf or the type's lowest value are never picked while another is left, and weigh nothing, also
+    where a whole column is masked (an expert that is switched off)."""
+    from moe_routers_b200 import ops
+
+    g = torch.Generator().manual_seed(t + e)
+    for low in (float("-inf"), torch.finfo(dtype).min):
+        a = torch.randn(t, e, generator=g).to(dtype)
+        a[:, 3] = low
+        a[:, e // 2:].masked_fill_(torch.rand(t, e - e // 2, generator=g) < 0.7, low)
+        a = a.cuda()
+        idx, w = ops.sinkhorn(a, 2)
+        ref_idx, ref_w, clear = _exact(a, 2, 10)
+        assert not (idx == 3).any() and torch.equal(idx.long()[clear], ref_idx[clear])
+        tol = 21 * 16 * 2.0 ** -24  # as above
+        torch.testing.assert_close(w.double()[clear], ref_w[clear], rtol=tol, atol=tol)
+    assert ops.read_status() == 0
+
+
 def test_sinkhorn_unaligned_logits():
     from moe_routers_b200 import ops
 
