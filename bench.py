@@ -621,7 +621,7 @@ def bench_strategies(torch, ops, dev, xs, w, capture, timed, med, event_us, peak
         _progress(f"  grouped FFN {n_exp} experts timed")
         variants = None
         if n_exp == 8:
-            # the same shape with one MMA-issuing thread, same box, same protocol
+            # the same shape with one MMA-issuing warp, same box, same protocol
             from moe_routers_b200._lib import lib as _l
             mode = _l.moe_set_gemm_mode(-1)
             _l.moe_set_gemm_mode(mode & ~2)

@@ -86,16 +86,17 @@ long long moe_launch_count(void);
  * after the call.  Measurement helper; no counterpart in the reference. */
 int moe_set_pdl(int enabled);
 
-/* Variants the grouped GEMM may use; every combination computes the same result bits, the default
- * (all on) is the fastest measured.  moe_set_gemm_mode(mode) replaces the set for launches issued
- * after the call (process-wide) and returns the previous one; a negative mode only reads it.
- * Measurement and test helper; no counterpart in the reference. */
+/* Variants of the grouped GEMM: one or two MMA-issuing warps (MOE_GEMM_TWO_ISSUERS), the same result
+ * bits either way; the default (two) is the faster one.  moe_set_gemm_mode(mode) replaces the set for
+ * launches issued after the call (process-wide) and returns the previous one; a negative mode only
+ * reads it.  Measurement and test helper; no counterpart in the reference.  The other bits are
+ * reserved: they chose among kernels that are gone, and are accepted and kept without effect. */
 enum {
-  MOE_GEMM_TWO_CTA = 1,       /* no effect: every call runs on the two-CTA kernel (tcgen05 cta_group::2) */
-  MOE_GEMM_TWO_ISSUERS = 2,   /* two MMA-issuing warps */
-  MOE_GEMM_TILE_PAIRS = 4,    /* no effect (a variant of a former one-CTA kernel), as the two below */
-  MOE_GEMM_M64 = 8,
-  MOE_GEMM_TWO_PRODUCERS = 16,
+  MOE_GEMM_TWO_CTA = 1,       /* reserved */
+  MOE_GEMM_TWO_ISSUERS = 2,
+  MOE_GEMM_TILE_PAIRS = 4,    /* reserved */
+  MOE_GEMM_M64 = 8,           /* reserved */
+  MOE_GEMM_TWO_PRODUCERS = 16,/* reserved */
   MOE_GEMM_ALL = 31
 };
 int moe_set_gemm_mode(int mode);

@@ -65,15 +65,13 @@ CASES = [
     ([24, 24, 7], 32, 64, "nk", "swiglu"),
     ([50, 3], 72, 48, "nk", "gelu"),
     ([50, 3], 64, 16, "nk", "swiglu"),
-    # average >= 512 rows per expert and 256 accumulator columns: work units are pairs of 128-row
-    # tiles sharing the weight stages (odd tile counts, empty experts, short last tiles included)
+    # several units of up to 256 rows per expert (empty and one-row experts, short last units included)
     ([600, 256, 300, 1000], 192, 256, "nk", None),
     ([600, 0, 150, 1300], 256, 512, "nk", "gelu"),
     ([385, 640, 1, 1030], 320, 256, "kn", None),
     ([600, 256, 300, 1000], 128, 128, "nk", "swiglu"),
     ([257, 513, 769, 564], 192, 256, "kn", "swiglu"),
-    # the same class of shapes on the two-CTA kernel: units of 512 rows, every remainder (1..3 tiles,
-    # partial tiles, a one-row expert, an empty expert), one k block, K not a multiple of 64, many units
+    # the same with one k block, K not a multiple of 64, rows just past whole units, many units
     ([129, 1280, 385, 900], 72, 256, "nk", None),
     ([1, 2047, 640, 0], 256, 256, "kn", "gelu"),
     ([1024], 64, 256, "nk", None),
@@ -198,8 +196,7 @@ def test_demo_pipeline_on_device(ops):
 def test_grouped_gemm_scattered_rows_equal_dense(ops, N, act, dtype, bias, counts):
     """`out_rows`: every result row stored at its own address.  With the addresses of a permuted
     buffer the result must be the dense result, row-permuted, bit for bit (same kernel arithmetic);
-    rows that no address points to stay untouched.  (The second set of counts runs on the two-CTA kernel
-    where the tile has 256 accumulator columns.)"""
+    rows that no address points to stay untouched."""
     K = 192
     off = _segments(counts)
     rows, e = int(off[-1]), len(counts)
@@ -225,38 +222,44 @@ def test_grouped_gemm_scattered_rows_equal_dense(ops, N, act, dtype, bias, count
 
 @pytest.mark.parametrize("counts,K,N,layout,act", [
     ([1045, 1037, 1009, 1021, 994, 1050, 1012, 1024], 512, 1024, "nk", "gelu"),
-    ([600, 0, 257, 1230], 200, 512, "kn", None),
+    ([600, 0, 257, 1230], 200, 512, "kn", None),           # K tail: 64 + 64 + 64 + 8
     ([2048, 1, 1023], 256, 256, "nk", "swiglu"),
+    ([40] * 300, 64, 256, "nk", None),                     # one stage per unit, several units per CTA pair
+    ([130, 7, 257, 64] * 40, 136, 256, "kn", "swiglu"),    # two stages, the second nearly empty
+    ([300, 31, 96] * 50, 320, 512, "nk", "silu"),          # three stages: units start with either warp
+    ([48] * 200, 1160, 256, "nk", None),                   # ten stages, more than the ring holds
 ])
 def test_grouped_gemm_variants_are_bit_identical(ops, counts, K, N, layout, act):
-    """Every kernel variant (two-CTA kernel with one or two MMA-issuing threads, two-tile units of one
-    CTA, single-tile units, M=64 last tiles on or off, one or two TMA warps) accumulates in the same
-    order, so the results must agree bit for bit, and a repeated call must reproduce itself."""
+    """One or two MMA-issuing warps issue the stages in the same order, so the results must agree bit for bit
+    however the stages of consecutive units fall to the warps, and a repeated call must reproduce itself.  The
+    result is also checked against fp32."""
     from moe_routers_b200._lib import lib
 
+    TWO_ISSUERS = 2
     off = _segments(counts)
     rows, e = int(off[-1]), len(counts)
     g = torch.Generator().manual_seed(len(counts) + K)
-    a = torch.randn(rows, K, generator=g).half().cuda()
+    a = torch.randn(rows, K, generator=g).half()
     n_w = 2 * N if act == "swiglu" else N
     shape = (e, n_w, K) if layout == "nk" else (e, K, n_w)
-    w = (torch.randn(*shape, generator=g) / K ** 0.5).half().cuda()
+    w = (torch.randn(*shape, generator=g) / K ** 0.5).half()
+    ref = _ref(a, w, off, layout, act)
+    a, w = a.cuda(), w.cuda()
     off_t = torch.from_numpy(off).cuda()
     before = lib.moe_set_gemm_mode(-1)
+    outs = []
     try:
-        outs = {}
-        for mode in (31, 31, 29, 30, 4 | 8 | 16, 8 | 16, 16, 0):
+        for mode in (31, 31, 31 & ~TWO_ISSUERS, 31 & ~TWO_ISSUERS, 31):
             lib.moe_set_gemm_mode(mode)
             out = ops.grouped_gemm(a, w, off_t, layout=layout, activation=act)
             torch.cuda.synchronize()
             assert ops.read_status() == 0
-            outs.setdefault(mode, []).append(out.view(torch.int16).cpu())
+            outs.append(out.cpu())
     finally:
         lib.moe_set_gemm_mode(before)
-    ref = outs[31][0]
-    for mode, got in outs.items():
-        for o in got:
-            assert torch.equal(o, ref), f"mode {mode} differs"
+    for i, o in enumerate(outs[1:]):
+        assert torch.equal(o.view(torch.int16), outs[0].view(torch.int16)), f"call {i + 1} differs"
+    np.testing.assert_allclose(outs[0].float().numpy(), ref, rtol=2e-2, atol=4e-3 * float(np.abs(ref).max()))
 
 
 @pytest.mark.parametrize("offsets", [
@@ -268,11 +271,11 @@ def test_grouped_gemm_variants_are_bit_identical(ops, counts, K, N, layout, act)
 def test_grouped_gemm_tolerates_invalid_offsets(ops, offsets, N):
     """The offsets come from another kernel; a caller that launches the GEMM on a stream that does not
     wait for that kernel hands it whatever the memory held.  Segments are forced into [0, rows] inside
-    the kernels, so such a call stays short (at most rows/128 + experts tiles), records no error and
-    writes only rows of the result buffer."""
+    the kernel, so such a call stays short (at most rows/256 + 1 units per expert and feature tile), records
+    no error and writes only rows of the result buffer."""
     import time
 
-    rows, K, e = (2400 if N == 256 else 1400), 128, 4  # 2400 rows: the two-CTA kernel where the total allows
+    rows, K, e = (2400 if N == 256 else 1400), 128, 4
     g = torch.Generator().manual_seed(1)
     a = torch.randn(rows, K, generator=g).half().cuda()
     w = (torch.randn(e, N, K, generator=g) / K ** 0.5).half().cuda()
@@ -291,8 +294,8 @@ def test_grouped_gemm_tolerates_invalid_offsets(ops, offsets, N):
 
 
 def test_grouped_gemm_sm_margin_same_result(ops):
-    """`sm_margin` leaves SMs free for a concurrent communication kernel: fewer persistent CTAs (or
-    CTA pairs) walk the same unit list, so the result must not change.  Shape on the two-CTA kernel."""
+    """`sm_margin` leaves SMs free for a concurrent communication kernel: fewer persistent CTA
+    pairs walk the same unit list, so the result must not change."""
     counts = [1100, 513, 0, 1200]
     off = _segments(counts)
     rows, e, K, N = int(off[-1]), len(counts), 256, 512
@@ -345,7 +348,7 @@ def test_consecutive_grouped_gemms_leave_room_for_another_stream(ops, experts, p
 @pytest.mark.parametrize("counts,K,N,layout,act,dtype", [
     ([1], 8, 16, "nk", None, torch.float16),                            # the smallest call
     ([31, 32, 33, 0, 255, 256, 257], 136, 272, "nk", "gelu", torch.float16),   # unit edges; a feature tile of 16
-    ([63, 64, 65, 127, 128, 129], 64, 464, "nk", None, torch.bfloat16),        # every token-box height; 208 features
+    ([63, 64, 65, 127, 128, 129], 64, 464, "nk", None, torch.bfloat16),        # short token boxes; 208 features in the second tile
     ([513, 1, 1793], 128, 240, "nk", None, torch.float16),              # evenly dealt units, fewer features than a tile
     ([17, 0, 300, 2], 200, 144, "nk", "swiglu", torch.float16),         # gate and up rows end inside a tile
     ([90, 160, 161], 192, 320, "kn", "swiglu", torch.bfloat16),
@@ -355,7 +358,7 @@ def test_consecutive_grouped_gemms_leave_room_for_another_stream(ops, experts, p
 @pytest.mark.parametrize("scattered", [False, True])
 def test_grouped_gemm_feature_major_edges(ops, counts, K, N, layout, act, dtype, scattered):
     """Tiles of 256 features x up to 256 tokens: sizes around every edge of the unit split (32-token steps,
-    256 tokens, token boxes of 16/32/64/128 rows), feature counts that fill no tile, K tails, dense and
+    256 tokens, token boxes of every multiple of 16 rows), feature counts that fill no tile, K tails, dense and
     scattered rows.  Bound: the result is rounded once to the storage type (2^-11 / 2^-8 of the value) after
     fp32 accumulation of K <= 200 products; the activations are smooth with slope <= 1.13 (times the gate's
     or up's magnitude, inside `scale`)."""
