@@ -1,5 +1,5 @@
 """The Sinkhorn kernel that keeps the matrix in registers, at the edges of its layouts: columns per lane,
-rows per lane, CTAs per cluster, and the shapes just outside of it, against the reference's iteration
+rows per lane, CTAs per cluster, and the two kernels behind it (shared memory of one cluster; a cooperative grid), against the reference's iteration
 (models/decoder_moe.py:92-123) in 64 bits."""
 import os
 import subprocess
@@ -20,7 +20,9 @@ CASES = [
     (4096, 64, 8, 10, torch.float32), (8192, 64, 2, 10, torch.float32), (8193, 64, 2, 10, torch.float32),
     (33, 65, 2, 10, torch.float32), (4096, 128, 4, 10, torch.float32), (4097, 128, 4, 3, torch.float32),
     (17, 129, 2, 10, torch.float32), (2048, 256, 8, 10, torch.float16), (2049, 255, 2, 3, torch.float32),
-    (100, 257, 2, 10, torch.float32),
+    # a cooperative grid: one CTA, two, and as many as a large matrix takes (16384 x 64: 128 CTAs)
+    (100, 257, 2, 10, torch.float32), (200, 257, 4, 10, torch.float32), (16384, 64, 2, 10, torch.float16),
+    (16387, 128, 4, 10, torch.bfloat16),
 ]
 
 
@@ -52,7 +54,7 @@ def test_sinkhorn_layout_edges(t, e, k, iters, dtype):
     # 2 * iters + 1 normalisations, each a sum (a few ulp), a product and a division in fp32
     tol = (2 * iters + 1) * 16 * 2.0 ** -24
     torch.testing.assert_close(w.double()[clear], ref_w[clear], rtol=tol, atol=tol)
-    # the router's own result types are these values, rounded once
+    # a second call on the same workspace, and the router's own result types: these values, rounded once
     ridx, rw = SinkhornRouter(iters=iters)(logits, k)
     assert ridx.dtype == torch.int64 and rw.dtype == dtype
     assert torch.equal(ridx, idx.long()) and torch.equal(rw, w.to(dtype))
@@ -76,6 +78,23 @@ def test_sinkhorn_masked_columns(t, e, dtype):
         assert not (idx == 3).any() and torch.equal(idx.long()[clear], ref_idx[clear])
         tol = 21 * 16 * 2.0 ** -24  # as above
         torch.testing.assert_close(w.double()[clear], ref_w[clear], rtol=tol, atol=tol)
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("t,e", [(300, 64), (70, 16), (40, 256), (300, 60), (200, 257), (8193, 64), (16384, 64)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_sinkhorn_nan(t, e, dtype):
+    """A NaN, a +inf or a row of -inf makes every sum NaN, as in the reference's arithmetic: all weights are NaN, and
+    the picks stay column numbers."""
+    from moe_routers_b200 import ops
+
+    for bad in (lambda a: a[5].fill_(float("-inf")), lambda a: a[5, 3:4].fill_(float("inf")),
+                lambda a: a[5, 3:4].fill_(float("nan"))):
+        a = torch.randn(t, e, generator=torch.Generator().manual_seed(t + e)).to(dtype).cuda()
+        bad(a)
+        idx, w = ops.sinkhorn(a, 2)
+        assert _exact(a, 2, 10)[1].isnan().all() and w.isnan().all()
+        assert ((idx >= 0) & (idx < e)).all()
     assert ops.read_status() == 0
 
 
