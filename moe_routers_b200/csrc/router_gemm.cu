@@ -369,11 +369,11 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
   if (threadIdx.x == kThreads - 32) {
     prefetch_tensormap(&tmap_x);
     prefetch_tensormap(&tmap_w);
-    // The tokens are an input of the whole route: nothing this library launches writes them.  Their
-    // boxes are requested into L2 here, ahead of the dependency wait below, so that with programmatic
-    // dependent launch the HBM reads of this route start under the tail of the kernel before it
-    // (in a sequence of routes: under the previous scatter's stores).  Only a hint: the copies into
-    // shared memory are issued after the wait and read whatever L2 then holds.
+    // The token boxes are requested into L2 here, ahead of the dependency wait below, so that with
+    // programmatic dependent launch the HBM reads of this route start under the tail of the kernel
+    // before it (in a sequence of routes: under the previous scatter's stores).  Only a hint, harmless
+    // also where that kernel is still writing the tokens (a GEMM in front of the route): L2 takes its
+    // stores, and the copies into shared memory are issued after the wait and read whatever L2 then holds.
     if (p.prefetch_x)
       for (int it = 0; it < nkb; ++it) tma_prefetch_l2_2d(&tmap_x, (kb0 + it) * kBlockK, block * kBlockTokens);
   }
