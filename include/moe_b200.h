@@ -197,6 +197,26 @@ int moe_pack_static(const void* x, int elem_bytes, const int32_t* idx, int token
                     int32_t* route_row, int32_t* device_status, void* stream);
 
 /*
+ * Strategy A's dense sweep: every expert over the same number of rows, in one launch and without an offsets array.
+ *   c[e * tokens + t] = act( a[row] @ W[e] ),  row = t with shared_rows (all experts read the same rows
+ *   a [tokens, K]), else e * tokens + t (a [experts * tokens, K]); c [experts * tokens, N]
+ * Replaces the loop over experts of the masked_matmul strategy (bench_router.py:438, bench_2gpu_pcie.py:123-171);
+ * types, layouts and limits as in moe_grouped_gemm.
+ */
+int moe_dense_experts(const void* a, const void* w, void* c, int experts, int tokens, int shared_rows, int K, int N,
+                      int w_layout, int64_t stride_w, int activation, int dtype, void* workspace,
+                      size_t workspace_bytes, void* stream);
+
+/*
+ * The gate-masked sum behind it: out[t] = sum_e g[t,e] * y[e * tokens + t], g[t,e] the gate of t's pick of e, 0 where
+ * e was not picked (the row is read and multiplied all the same), accumulated in fp32 in ascending e.
+ *   y [experts * tokens, d] fp16/bf16, idx [tokens, top_k] int32, gates [tokens, top_k] float32, out [tokens, d]
+ * Limits: experts <= 8, top_k <= 8, d a multiple of 8, y and out 16-byte aligned.
+ */
+int moe_combine_dense(const void* y, int dtype, const int32_t* idx, const float* gates, int tokens, int d, int experts,
+                      int top_k, void* out, void* stream);
+
+/*
  * Gate-weighted un-permute and sum over the top_k picks:
  *   out[t] = sum_j gates[t,j] * y[route_row[t*top_k + j]]   (fp32 accumulate)
  * Replaces: `expert(x_e) * w_e` + index_add_ (models/decoder_moe.py:270-271).

@@ -36,12 +36,14 @@ __device__ __forceinline__ uint32_t pack2<__nv_bfloat162>(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Vector path: d % 8 == 0 and 16-byte aligned bases.
-template <typename T2, int TOPK, bool SPLIT>
+// Vector path: d % 8 == 0 and 16-byte aligned bases.  DENSE: the rows are those of all experts (`top_k_rt` of them,
+// expert e's row of token t at e * tokens + t), `route_row` holds the token's `picks` experts, and a row's gate is
+// that of the pick of its expert, or 0.
+template <typename T2, int TOPK, bool SPLIT, bool DENSE = false>
 __global__ void __launch_bounds__(kWarps * 32)
 combine_vec_kernel(const uint4* __restrict__ y, const float* __restrict__ gates,
                    const int32_t* __restrict__ route_row, uint4* __restrict__ out, int tokens,
-                   int n_vec_total, int part_vec, int top_k_rt, int total_rows) {
+                   int n_vec_total, int part_vec, int top_k_rt, int total_rows, int picks = 0) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * kWarps + (threadIdx.x >> 5);
   // launched with programmatic stream serialisation: everything in global memory is touched after this
@@ -55,8 +57,16 @@ combine_vec_kernel(const uint4* __restrict__ y, const float* __restrict__ gates,
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     if (j < top_k) {
-      int row = route_row[(size_t)t * top_k + j];
-      g[j] = gates[(size_t)t * top_k + j];
+      int row;
+      if constexpr (DENSE) {
+        row = j * tokens + t;
+        g[j] = 0.f;
+        for (int i = 0; i < picks; ++i)
+          if (__ldg(route_row + (size_t)t * picks + i) == j) g[j] += __ldg(gates + (size_t)t * picks + i);
+      } else {
+        row = route_row[(size_t)t * top_k + j];
+        g[j] = gates[(size_t)t * top_k + j];
+      }
       if ((unsigned)row >= (unsigned)total_rows) { row = 0; g[j] = 0.f; }  // never read out of bounds
       src[j] = y + (size_t)row * n_vec_total;
     }
@@ -124,6 +134,38 @@ combine_scalar_kernel(const T* __restrict__ y, const float* __restrict__ gates,
   }
 }
 
+// The columns of a token are halved, down to one load per lane and row, until there are two CTAs for every SM.
+inline int part_of(int n_vec, int grid) {
+  int part = (n_vec + 127) & ~127;
+  while (part > 32 && (long long)grid * ((n_vec + part - 1) / part) < kFillCtas) part = ((part / 2) + 31) & ~31;
+  return part;
+}
+template <typename Kernel>
+int launch_split(Kernel kernel, const uint4* y, const float* gates, const int32_t* rows, uint4* out, int tokens, int n_vec,
+                 int part, int top_k, int total_rows, int picks, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((tokens + kWarps - 1) / kWarps, (n_vec + part - 1) / part, 1);
+  cfg.blockDim = dim3(kWarps * 32, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, y, gates, rows, out, tokens, n_vec, part, top_k, total_rows, picks);
+  if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "combine_kernel: %s", cudaGetErrorString(e));
+  note_launch();
+  return MOE_OK;
+}
+
+template <typename T2>
+int launch_combine_dense(const void* y, const int32_t* idx, const float* gates, int tokens, int d, int experts, int top_k,
+                         void* out, cudaStream_t s) {
+  const int n_vec = d / 8;
+  return launch_split(combine_vec_kernel<T2, 0, true, true>, static_cast<const uint4*>(y), gates, idx, static_cast<uint4*>(out),
+                      tokens, n_vec, part_of(n_vec, (tokens + kWarps - 1) / kWarps), experts, experts * tokens, top_k, s);
+}
+
 template <typename T, typename T2>
 int launch_combine(const void* y, const float* gates, const int32_t* route_row, int tokens, int d,
                    int top_k, void* out, cudaStream_t s) {
@@ -141,25 +183,11 @@ int launch_combine(const void* y, const float* gates, const int32_t* route_row, 
         combine_vec_kernel<T2, 0, false><<<grid, kWarps * 32, 0, s>>>(yy, gates, route_row, oo, tokens, n_vec, n_vec, top_k, total_rows);
       return check_launch("combine_kernel");
     }
-    // Few tokens: the columns are halved, down to one load per lane and row, until there are two CTAs for every
-    // SM, and the kernel sets itself up under the GEMM in front of it (4 x 4096: 5.5 -> 1.6 us; 600 x 2048, k 4:
-    // 5.1 -> 4.5; the same code with whole rows was 6 % slower at 4096 and 16387 tokens, hence the template).
-    int part = (n_vec + 127) & ~127;
-    while (part > 32 && (long long)grid * ((n_vec + part - 1) / part) < kFillCtas) part = ((part / 2) + 31) & ~31;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, (n_vec + part - 1) / part, 1);
-    cfg.blockDim = dim3(kWarps * 32, 1, 1);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, top_k == 2 ? combine_vec_kernel<T2, 2, true> : combine_vec_kernel<T2, 0, true>,
-                                             yy, gates, route_row, oo, tokens, n_vec, part, top_k, total_rows);
-    if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "combine_kernel: %s", cudaGetErrorString(e));
-    note_launch();
-    return MOE_OK;
+    // Few tokens: the columns are dealt to several CTAs, and the kernel sets itself up under the GEMM in front of it
+    // (4 x 4096: 5.5 -> 1.6 us; 600 x 2048, k 4: 5.1 -> 4.5; the same code with whole rows was 6 % slower at 4096 and
+    // 16387 tokens, hence the template).
+    return launch_split(top_k == 2 ? combine_vec_kernel<T2, 2, true> : combine_vec_kernel<T2, 0, true>, yy, gates, route_row, oo,
+                        tokens, n_vec, part_of(n_vec, grid), top_k, total_rows, 0, s);
   } else {
     combine_scalar_kernel<T><<<grid, kWarps * 32, 0, s>>>(static_cast<const T*>(y), gates, route_row,
                                                          static_cast<T*>(out), tokens, d, top_k, total_rows);
@@ -182,5 +210,23 @@ extern "C" int moe_combine(const void* y, int dtype, const float* gates, const i
     case MOE_F16: return launch_combine<__half, __half2>(y, gates, route_row, tokens, d, top_k, out, s);
     case MOE_BF16: return launch_combine<__nv_bfloat16, __nv_bfloat162>(y, gates, route_row, tokens, d, top_k, out, s);
     default: return fail(MOE_ERR_ARG, "moe_combine: dtype must be fp16 or bf16");
+  }
+}
+
+extern "C" int moe_combine_dense(const void* y, int dtype, const int32_t* idx, const float* gates, int tokens, int d,
+                                 int experts, int top_k, void* out, void* stream) {
+  using namespace moe;
+  if (tokens < 0 || d <= 0 || d % 8 != 0) return fail(MOE_ERR_ARG, "moe_combine_dense: bad shape");
+  if (experts < 1 || experts > 8) return fail(MOE_ERR_UNSUPPORTED, "moe_combine_dense: experts must be in [1,8], got %d", experts);
+  if (top_k < 1 || top_k > 8) return fail(MOE_ERR_UNSUPPORTED, "moe_combine_dense: top_k must be in [1,8], got %d", top_k);
+  if (tokens == 0) return MOE_OK;
+  if (!y || !idx || !gates || !out) return fail(MOE_ERR_ARG, "moe_combine_dense: null pointer");
+  if ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15)
+    return fail(MOE_ERR_ARG, "moe_combine_dense: y and out must be 16-byte aligned");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case MOE_F16: return launch_combine_dense<__half2>(y, idx, gates, tokens, d, experts, top_k, out, s);
+    case MOE_BF16: return launch_combine_dense<__nv_bfloat162>(y, idx, gates, tokens, d, experts, top_k, out, s);
+    default: return fail(MOE_ERR_ARG, "moe_combine_dense: dtype must be fp16 or bf16");
   }
 }

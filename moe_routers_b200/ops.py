@@ -370,3 +370,48 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, *, lay
                                    _DTYPE_CODE[a.dtype], int(sm_margin),
                                    ws.data_ptr(), ws.numel(), _stream()))
     return c
+
+
+def dense_experts(a: torch.Tensor, w: torch.Tensor, tokens: int, *, activation: Optional[str] = None,
+                  out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """c[e * tokens + t] = act(a[row] @ W[e].T) for every expert and token: row = t where `a` has `tokens` rows, which
+    all experts read, else e * tokens + t.  w [E, N, K]; fp16 or bf16."""
+    _require_cuda(a, w)
+    if a.dtype not in (torch.float16, torch.bfloat16) or w.dtype != a.dtype:
+        raise RuntimeError("grouped_gemm: a and w must both be fp16 or both bf16")
+    if w.dim() != 3:
+        raise RuntimeError("grouped_gemm: w must be [E, N, K]")
+    a = a.contiguous()
+    w = w.contiguous()
+    e, n_w, k_dim = w.shape
+    if a.size(1) != k_dim:
+        raise RuntimeError("grouped_gemm: inner dimensions differ")
+    if a.size(0) not in (tokens, e * tokens):
+        raise RuntimeError("dense_experts: a must have tokens or experts * tokens rows")
+    act = _ACT[activation]
+    n_out = n_w // 2 if act == _lib.MOE_ACT_SWIGLU else n_w
+    dev = a.get_device()
+    with _on(dev):
+        ws = _workspace(dev, 1, e, 1)
+        c = out if out is not None else empties(dev, ((a.dtype, e * tokens, n_out),))[0]
+        check(lib.moe_dense_experts(a.data_ptr(), w.data_ptr(), c.data_ptr(), e, tokens, int(a.size(0) == tokens), k_dim, n_out,
+                                    _lib.MOE_W_NK, w.stride(0), act, _DTYPE_CODE[a.dtype], ws.data_ptr(), ws.numel(),
+                                    _stream()))
+    return c
+
+
+def combine_dense(y: torch.Tensor, idx: torch.Tensor, gates: torch.Tensor, experts: int) -> torch.Tensor:
+    """out[t] = sum_e g[t, e] * y[e * T + t] with the gate of t's pick of expert e, 0 for the experts not picked."""
+    _require_cuda(y, idx, gates)
+    if y.dtype not in (torch.float16, torch.bfloat16):
+        raise RuntimeError("y must be fp16 or bf16")
+    y = y.contiguous()
+    idx = idx.to(torch.int32).contiguous()
+    gates = gates.to(torch.float32).contiguous()
+    t, d = y.size(0) // experts, y.size(1)
+    dev = y.get_device()
+    with _on(dev):
+        out, = empties(dev, ((y.dtype, t, d),))
+        check(lib.moe_combine_dense(y.data_ptr(), _DTYPE_CODE[y.dtype], idx.data_ptr(), gates.data_ptr(), t, d, int(experts),
+                                    idx.size(1), out.data_ptr(), _stream()))
+    return out
