@@ -379,6 +379,11 @@ __global__ void __launch_bounds__(kRegThreads, 1) sinkhorn_regs_kernel(const SPa
   // remote stores need every CTA of the cluster running with its barriers initialised: arrive now, wait
   // before the first store
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  // Launched with programmatic stream serialisation: placing a cluster and everything above go on while the kernel in
+  // front (a router GEMM, another call's Sinkhorn on 16 of the other SMs) is running; nothing in global memory is
+  // touched before the wait.  Calls one behind the other, 4096 x 64: 22.55 -> 20.75 us.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   // ---- K = exp(s - rowmax), s = (logits / temperature) rounded to the logits dtype ----
   const int rg = lane / LPR, c0 = (lane % LPR) * kRegCols;
@@ -613,14 +618,17 @@ int launch_sinkhorn_regs(SParams p, cudaStream_t s) {
     cfg.blockDim = dim3(kRegThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (ctas > 8 && !places_wide_cluster(kernel, cfg)) continue;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
     e = cudaLaunchKernelEx(&cfg, kernel, static_cast<const SParams>(p));
     if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "sinkhorn_regs_kernel: %s", cudaGetErrorString(e));
     note_launch();
