@@ -106,6 +106,11 @@ int moe_set_gemm_mode(int mode);
  * which bounded wait gave up (see moe_last_error). */
 int moe_read_status(const void* workspace, void* stream, int* status_host);
 
+/* Copy `n` <= 1025 int32 words (segment offsets that the host already knows) to device memory in stream order.
+ * They travel as arguments of a small kernel, so `host` may be reused at once and no pinned buffer is needed.
+ * Replaces the problem-size arrays that kernels/grouped_ffn.cu:84-121 uploads. */
+int moe_store_offsets(const int32_t* host, int n, int32_t* device, void* stream);
+
 /*
  * Top-k selection with softmax gates over the selected logits.
  * Replaces: fused_select_cuda.forward(logits, k) as called by CUDATopKRouter

@@ -32,6 +32,7 @@ SIGNATURES = {
     "moe_launch_count": (C.c_longlong, []),
     "moe_set_pdl": (_i, [_i]),
     "moe_set_gemm_mode": (_i, [_i]),
+    "moe_store_offsets": (_i, [C.POINTER(C.c_int32), _i, _p, _p]),
     "moe_topk_select": (_i, [_p, _i, _i, _i, _i, _p, _p, _p]),
     "moe_pack": (_i, [_p, _i, _p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p, _sz, _p]),
     "moe_fused_select": (_i, [_p, _i, _p, _i, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _sz, _p]),

@@ -60,7 +60,8 @@ def _host_stamp() -> str:
 
 
 def _host_fresh(stamp: str) -> bool:
-    if not os.path.exists(HOST_PATH) or os.path.getmtime(HOST_PATH) < os.path.getmtime(HOST_SRC):
+    if not os.path.exists(HOST_PATH) or os.path.getmtime(HOST_PATH) < max(
+            os.path.getmtime(p) for p in [HOST_SRC] + glob.glob(os.path.join(INCLUDE, "*.h"))):
         return False
     try:
         with open(HOST_STAMP) as f:

@@ -134,3 +134,36 @@ extern "C" int moe_device_pci_bus_id(int device, char* out, int len) {
   if (e != cudaSuccess) return moe::fail(MOE_ERR_DEVICE, "moe_device_pci_bus_id: %s", cudaGetErrorString(e));
   return MOE_OK;
 }
+
+namespace moe {
+namespace {
+
+constexpr int kMaxOffsets = 1025;  // experts + 1
+template <int N>
+struct Words {
+  int32_t v[N];
+};
+template <int N>
+__global__ void __launch_bounds__(128) store_words_kernel(const __grid_constant__ Words<N> words, int n, int32_t* out) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM behind sets itself up and waits
+  for (int i = threadIdx.x; i < n; i += (int)blockDim.x) out[i] = words.v[i];
+}
+template <int N>
+int store_words(const int32_t* host, int n, int32_t* device, cudaStream_t s) {
+  Words<N> w;
+  memcpy(w.v, host, n * sizeof(int32_t));
+  store_words_kernel<N><<<1, 128, 0, s>>>(w, n, device);
+  return check_launch("store_words_kernel");
+}
+
+}  // namespace
+}  // namespace moe
+
+extern "C" int moe_store_offsets(const int32_t* host, int n, int32_t* device, void* stream) {
+  using namespace moe;
+  if (n < 0 || (n > 0 && (!host || !device))) return fail(MOE_ERR_ARG, "moe_store_offsets: bad argument");
+  if (n > kMaxOffsets) return fail(MOE_ERR_UNSUPPORTED, "moe_store_offsets: at most %d words, got %d", kMaxOffsets, n);
+  if (n == 0) return MOE_OK;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return n <= 72 ? store_words<72>(host, n, device, s) : store_words<kMaxOffsets>(host, n, device, s);
+}

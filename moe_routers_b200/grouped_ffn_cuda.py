@@ -48,6 +48,10 @@ def grouped_ffn_forward(inputs: List[torch.Tensor], weights: List[torch.Tensor])
         return []
     if len(inputs) != len(weights):
         raise RuntimeError("grouped_ffn_forward: inputs and weights must have the same length")
+    if inputs[0].is_cuda:
+        out = ops.grouped_lists(inputs, weights)
+        if out is not None:
+            return out
     for a, w in zip(inputs, weights):
         if not (a.is_cuda and w.is_cuda):
             raise RuntimeError("inputs must be CUDA")

@@ -129,9 +129,7 @@ class MoELayer(torch.nn.Module):
         if track:
             ev[1].record()
         w13, w2 = self._stacked_weights()
-        h = ops.grouped_gemm(packed, w13, offsets, layout="nk", activation="swiglu")
-        y = ops.grouped_gemm(h, w2, offsets, layout="nk")
-        out = ops.combine(y, gates, route_row, k)
+        out = ops.expert_ffn(packed, w13, w2, offsets, gates, route_row, k, activation="swiglu")
         if track:
             ev[2].record()
             torch.cuda.synchronize()

@@ -9,11 +9,12 @@ rejected.
 from __future__ import annotations
 
 import contextlib
+import ctypes
 from typing import Optional
 
 import torch
 
-from . import _lib
+from . import _host, _lib
 from ._host import empties
 from ._lib import check, lib
 
@@ -59,10 +60,14 @@ def _workspace(index: int, tokens: int, experts: int, top_k: int) -> torch.Tenso
     return ws
 
 
+# The operators that _host runs as one native call where their arguments are plain; the functions below take the rest.
+_host.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value
+            for name in ("moe_workspace_bytes", "moe_route_fused", "moe_fused_select", "moe_sinkhorn", "moe_sinkhorn_router",
+                         "moe_grouped_gemm", "moe_combine", "moe_store_offsets")}, _workspaces, _workspace, check)
+
+
 def read_status(device: Optional[torch.device] = None) -> int:
     """Synchronise the current stream and raise if a kernel recorded an error."""
-    import ctypes
-
     device = device or torch.device("cuda", torch.cuda.current_device())
     ws = workspace(device, 1, 1, 1)
     out = ctypes.c_int(0)
@@ -185,6 +190,11 @@ def fused_select(logits: torch.Tensor, x: torch.Tensor, experts: int, top_k: int
     """Select + count + scan + pack from given logits in two launches.
     Returns (idx, gates, counts, offsets, packed, row_route, route_row); `out` may be the tuple a
     previous call returned, to reuse its buffers."""
+    if out is None and x.is_cuda:
+        dev = _current_device()
+        o = _host.fused_select(dev, _raw_stream(dev), logits, x, experts, top_k)
+        if o is not None:
+            return o
     _require_cuda(logits, x)
     if logits.dtype not in _DTYPE_CODE:
         raise RuntimeError("logits must be fp16/bf16/fp32")
@@ -256,6 +266,11 @@ def route_fused(x: torch.Tensor, w_router: torch.Tensor, top_k: int, *, skew_exp
     until the next route on that stream.  `out` may carry pre-allocated
     tensors from a previous call to avoid re-allocation.
     """
+    if out is None and x.is_cuda:
+        dev = _current_device()
+        o = _host.route(dev, _raw_stream(dev), x, w_router, top_k, skew_experts, skew_bias, bool(return_logits))
+        if o is not None:
+            return o
     _require_cuda(x, w_router)
     if x.dtype not in (torch.float16, torch.bfloat16) or w_router.dtype != x.dtype:
         raise RuntimeError("x and the router weight must both be fp16 (Half) or both bf16")
@@ -286,17 +301,24 @@ def route_fused(x: torch.Tensor, w_router: torch.Tensor, top_k: int, *, skew_exp
 def sinkhorn(logits: torch.Tensor, top_k: int, *, iters: int = 10, epsilon: float = 1e-6,
              temperature: float = 1.0):
     """Sinkhorn-balanced top-k: (idx int32 [T,k], gates float32 [T,k])."""
-    return _sinkhorn(lib.moe_sinkhorn, torch.int32, torch.float32, logits, top_k, iters, epsilon, temperature)
+    return _sinkhorn(False, logits, top_k, iters, epsilon, temperature)
 
 
 def sinkhorn_router(logits: torch.Tensor, top_k: int, *, iters: int = 10, epsilon: float = 1e-6,
                     temperature: float = 1.0):
     """The same as the router plug-in returns it: (idx int64 [T,k], weights [T,k] in the logits' type)."""
-    return _sinkhorn(lib.moe_sinkhorn_router, torch.int64, logits.dtype, logits, top_k, iters, epsilon, temperature)
+    return _sinkhorn(True, logits, top_k, iters, epsilon, temperature)
 
 
-def _sinkhorn(entry, idx_dtype, gate_dtype, logits, top_k, iters, epsilon, temperature):
+def _sinkhorn(router: bool, logits, top_k, iters, epsilon, temperature):
+    if logits.is_cuda:
+        dev = _current_device()
+        o = _host.sinkhorn(dev, _raw_stream(dev), router, logits, top_k, iters, epsilon, temperature)
+        if o is not None:
+            return o
     _require_cuda(logits)
+    entry, idx_dtype, gate_dtype = ((lib.moe_sinkhorn_router, torch.int64, logits.dtype) if router else
+                                    (lib.moe_sinkhorn, torch.int32, torch.float32))
     if logits.dim() != 2:
         raise ValueError("SinkhornRouter expects logits of shape [tokens, experts]")
     if logits.dtype not in _DTYPE_CODE:
@@ -415,3 +437,26 @@ def combine_dense(y: torch.Tensor, idx: torch.Tensor, gates: torch.Tensor, exper
         check(lib.moe_combine_dense(y.data_ptr(), _DTYPE_CODE[y.dtype], idx.data_ptr(), gates.data_ptr(), t, d, int(experts),
                                     idx.size(1), out.data_ptr(), _stream()))
     return out
+
+
+def expert_ffn(rows: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, offsets: torch.Tensor, gates: torch.Tensor,
+               route_row: torch.Tensor, top_k: int, *, activation: Optional[str]) -> torch.Tensor:
+    """Two grouped GEMMs ([E, N, K] weights, the activation after the first) over the packed rows, then the
+    gate-weighted combine."""
+    if rows.is_cuda:
+        dev = _current_device()
+        o = _host.expert_ffn(dev, _raw_stream(dev), rows, w1, w2, offsets, _ACT[activation], gates, route_row, top_k)
+        if o is not None:
+            return o
+    h = grouped_gemm(rows, w1, offsets, layout="nk", activation=activation)
+    y = grouped_gemm(h, w2, offsets, layout="nk")
+    return combine(y, gates, route_row, top_k)
+
+
+def grouped_lists(inputs: list, weights: list) -> Optional[list]:
+    """[M_i, K] inputs times [K, N] weights, pair by pair, where both lists are consecutive views of one fp16 buffer
+    each; None, with nothing done, where they are not or a stream is being captured."""
+    dev = _current_device()
+    if torch.cuda.is_current_stream_capturing():
+        return None  # (the general path uploads the offsets in a way that a capture refuses, as it always has)
+    return _host.grouped_lists(dev, _raw_stream(dev), inputs, weights)

@@ -38,9 +38,7 @@ def route(strategy: str, x: torch.Tensor, w_router: torch.Tensor, top_k: int, *,
 
 def moe_forward(r: dict, w1: torch.Tensor, w2: torch.Tensor, top_k: int, activation: str = "gelu") -> torch.Tensor:
     """Sparse layer output from a routing with a packed buffer: grouped FFN + gate-weighted combine."""
-    h = ops.grouped_gemm(r["packed"], w1, r["offsets"], layout="nk", activation=activation)
-    y = ops.grouped_gemm(h, w2, r["offsets"], layout="nk")
-    return ops.combine(y, r["gates"], r["route_row"], top_k)
+    return ops.expert_ffn(r["packed"], w1, w2, r["offsets"], r["gates"], r["route_row"], top_k, activation=activation)
 
 
 def masked_matmul_forward(x: torch.Tensor, r: dict, w1: torch.Tensor, w2: torch.Tensor, top_k: int,
