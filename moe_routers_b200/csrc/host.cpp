@@ -293,10 +293,10 @@ PyObject* route(PyObject*, PyObject* const* args, Py_ssize_t n) {
   THPObjectPtr out(PyDict_New());
   if (!out) return nullptr;
   static PyObject* const names[] = {
-      PyUnicode_InternFromString("idx"), PyUnicode_InternFromString("gates"), PyUnicode_InternFromString("packed"),
-      PyUnicode_InternFromString("counts"), PyUnicode_InternFromString("offsets"), PyUnicode_InternFromString("row_route"),
+      PyUnicode_InternFromString("idx"), PyUnicode_InternFromString("gates"), PyUnicode_InternFromString("counts"),
+      PyUnicode_InternFromString("offsets"), PyUnicode_InternFromString("packed"), PyUnicode_InternFromString("row_route"),
       PyUnicode_InternFromString("route_row"), PyUnicode_InternFromString("logits")};
-  at::Tensor* const tensors[] = {&r.idx, &r.gates, &r.packed, &r.counts, &r.offsets, &r.row_route, &r.route_row, &r.logits};
+  at::Tensor* const tensors[] = {&r.idx, &r.gates, &r.counts, &r.offsets, &r.packed, &r.row_route, &r.route_row, &r.logits};
   for (int i = 0; i < (with_logits ? 8 : 7); ++i) {
     THPObjectPtr v(THPVariable_Wrap(std::move(*tensors[i])));
     if (!v || PyDict_SetItem(out.get(), names[i], v.get()) != 0) return nullptr;
