@@ -202,6 +202,17 @@ int moe_pack_static(const void* x, int elem_bytes, const int32_t* idx, int token
                     int32_t* route_row, int32_t* device_status, void* stream);
 
 /*
+ * The expert layer on packed rows in one call: hidden = act(a @ W1[e]), y = hidden @ W2[e], out = the gate-weighted sum of
+ * moe_combine; w1 [experts, h (SwiGLU: 2 h), d], w2 [experts, d_out, h], both MOE_W_NK and dense; hidden [rows, h] and
+ * y [rows, d_out] are scratch.  Replaces the per-expert loops and the combine of models/decoder_moe.py:256-273.  Knowing both
+ * GEMMs, it lets the second one fetch its first weights under the end of the first; otherwise as the three calls.
+ */
+int moe_expert_ffn(const void* a, const void* w1, void* hidden, const void* w2, void* y, const int32_t* offsets,
+                   int experts, int rows, int d, int h, int d_out, int activation, const float* gates,
+                   const int32_t* route_row, int top_k, void* out, int dtype, void* workspace, size_t workspace_bytes,
+                   void* stream);
+
+/*
  * Strategy A's dense sweep: every expert over the same number of rows, in one launch and without an offsets array.
  *   c[e * tokens + t] = act( a[row] @ W[e] ),  row = t with shared_rows (all experts read the same rows
  *   a [tokens, K]), else e * tokens + t (a [experts * tokens, K]); c [experts * tokens, N]

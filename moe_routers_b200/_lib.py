@@ -55,6 +55,7 @@ SIGNATURES = {
     "moe_sinkhorn_router": (_i, [_p, _i, _i, _i, _i, _i, _f, _f, _p, _p, _p, _sz, _p]),
     "moe_grouped_gemm": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _i, C.c_int64, _i, _p, _p, _i, _i, _p, _sz, _p]),
     "moe_grouped_gemm_rows": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _i, C.c_int64, _i, _p, _p, _i, _i, _p, _sz, _p]),
+    "moe_expert_ffn": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _p, _i, _p, _i, _p, _sz, _p]),
     "moe_dense_experts": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, C.c_int64, _i, _i, _p, _sz, _p]),
     "moe_combine_dense": (_i, [_p, _i, _p, _p, _i, _i, _i, _i, _p, _p]),
     "moe_pack_scatter_to": (_i, [_p, _i, _p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p, _sz, _p]),

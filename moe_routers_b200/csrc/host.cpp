@@ -141,7 +141,7 @@ struct Api {
   decltype(&moe_sinkhorn) sinkhorn;
   decltype(&moe_sinkhorn_router) sinkhorn_router;
   decltype(&moe_grouped_gemm) grouped_gemm;
-  decltype(&moe_combine) combine;
+  decltype(&moe_expert_ffn) expert_ffn;
   decltype(&moe_store_offsets) store_offsets;
 };
 Api api;
@@ -159,7 +159,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
       {"moe_sinkhorn", reinterpret_cast<void**>(&api.sinkhorn)},
       {"moe_sinkhorn_router", reinterpret_cast<void**>(&api.sinkhorn_router)},
       {"moe_grouped_gemm", reinterpret_cast<void**>(&api.grouped_gemm)},
-      {"moe_combine", reinterpret_cast<void**>(&api.combine)},
+      {"moe_expert_ffn", reinterpret_cast<void**>(&api.expert_ffn)},
       {"moe_store_offsets", reinterpret_cast<void**>(&api.store_offsets)},
   };
   for (const auto& e : entries) {
@@ -394,18 +394,11 @@ PyObject* expert_ffn(PyObject*, PyObject* const* args, Py_ssize_t n) {
   {
     WithoutGil released;
     hidden = c.make({rows, h}, a->scalar_type());
-    rc = api.grouped_gemm(a->data_ptr(), w1->data_ptr(), hidden.data_ptr(), data<int32_t>(*offsets), (int)e, (int)rows, (int)d, (int)h,
-                          MOE_W_NK, w1->stride(0), act, nullptr, nullptr, type, 0, c.ws, c.ws_bytes, c.stream);
-    if (rc == MOE_OK) {
-      y = c.make({rows, d2}, a->scalar_type());
-      rc = api.grouped_gemm(hidden.data_ptr(), w2->data_ptr(), y.data_ptr(), data<int32_t>(*offsets), (int)e, (int)rows, (int)h, (int)d2,
-                            MOE_W_NK, w2->stride(0), MOE_ACT_NONE, nullptr, nullptr, type, 0, c.ws, c.ws_bytes, c.stream);
-    }
-    if (rc == MOE_OK) {
-      const int64_t t = rows / k;
-      out = c.make({t, d2}, a->scalar_type());
-      rc = api.combine(y.data_ptr(), type, data<float>(*gates), data<int32_t>(*route_row), (int)t, (int)d2, k, out.data_ptr(), c.stream);
-    }
+    y = c.make({rows, d2}, a->scalar_type());
+    out = c.make({rows / k, d2}, a->scalar_type());
+    rc = api.expert_ffn(a->data_ptr(), w1->data_ptr(), hidden.data_ptr(), w2->data_ptr(), y.data_ptr(), data<int32_t>(*offsets), (int)e,
+                        (int)rows, (int)d, (int)h, (int)d2, act, data<float>(*gates), data<int32_t>(*route_row), k, out.data_ptr(),
+                        type, c.ws, c.ws_bytes, c.stream);
   }
   checked(rc);
   return THPVariable_Wrap(std::move(out));

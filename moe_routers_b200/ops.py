@@ -63,7 +63,7 @@ def _workspace(index: int, tokens: int, experts: int, top_k: int) -> torch.Tenso
 # The operators that _host runs as one native call where their arguments are plain; the functions below take the rest.
 _host.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value
             for name in ("moe_workspace_bytes", "moe_route_fused", "moe_fused_select", "moe_sinkhorn", "moe_sinkhorn_router",
-                         "moe_grouped_gemm", "moe_combine", "moe_store_offsets")}, _workspaces, _workspace, check)
+                         "moe_grouped_gemm", "moe_expert_ffn", "moe_store_offsets")}, _workspaces, _workspace, check)
 
 
 def read_status(device: Optional[torch.device] = None) -> int:
