@@ -47,7 +47,7 @@ combine_vec_kernel(const uint4* __restrict__ y, const float* __restrict__ gates,
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * kWarps + (threadIdx.x >> 5);
   // launched with programmatic stream serialisation: everything in global memory is touched after this
-  if (SPLIT) asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (t >= tokens) return;
   const int v_begin = SPLIT ? blockIdx.y * part_vec : 0;  // this warp's 16-byte pieces of the row
   const int n_vec = SPLIT ? min(n_vec_total, v_begin + part_vec) : n_vec_total;
@@ -141,7 +141,7 @@ inline int part_of(int n_vec, int grid) {
   return part;
 }
 template <typename Kernel>
-int launch_split(Kernel kernel, const uint4* y, const float* gates, const int32_t* rows, uint4* out, int tokens, int n_vec,
+int launch_vec(Kernel kernel, const uint4* y, const float* gates, const int32_t* rows, uint4* out, int tokens, int n_vec,
                  int part, int top_k, int total_rows, int picks, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((tokens + kWarps - 1) / kWarps, (n_vec + part - 1) / part, 1);
@@ -162,7 +162,7 @@ template <typename T2>
 int launch_combine_dense(const void* y, const int32_t* idx, const float* gates, int tokens, int d, int experts, int top_k,
                          void* out, cudaStream_t s) {
   const int n_vec = d / 8;
-  return launch_split(combine_vec_kernel<T2, 0, true, true>, static_cast<const uint4*>(y), gates, idx, static_cast<uint4*>(out),
+  return launch_vec(combine_vec_kernel<T2, 0, true, true>, static_cast<const uint4*>(y), gates, idx, static_cast<uint4*>(out),
                       tokens, n_vec, part_of(n_vec, (tokens + kWarps - 1) / kWarps), experts, experts * tokens, top_k, s);
 }
 
@@ -176,17 +176,13 @@ int launch_combine(const void* y, const float* gates, const int32_t* route_row, 
     const uint4* yy = static_cast<const uint4*>(y);
     uint4* oo = static_cast<uint4*>(out);
     const int n_vec = d / 8;
-    if (grid >= kFillCtas) {
-      if (top_k == 2)
-        combine_vec_kernel<T2, 2, false><<<grid, kWarps * 32, 0, s>>>(yy, gates, route_row, oo, tokens, n_vec, n_vec, top_k, total_rows);
-      else
-        combine_vec_kernel<T2, 0, false><<<grid, kWarps * 32, 0, s>>>(yy, gates, route_row, oo, tokens, n_vec, n_vec, top_k, total_rows);
-      return check_launch("combine_kernel");
-    }
-    // Few tokens: the columns are dealt to several CTAs, and the kernel sets itself up under the GEMM in front of it
-    // (4 x 4096: 5.5 -> 1.6 us; 600 x 2048, k 4: 5.1 -> 4.5; the same code with whole rows was 6 % slower at 4096 and
-    // 16387 tokens, hence the template).
-    return launch_split(top_k == 2 ? combine_vec_kernel<T2, 2, true> : combine_vec_kernel<T2, 0, true>, yy, gates, route_row, oo,
+    // Set up under the GEMM in front of it in either form (layer of 3330 x 768: 67.5 -> 65.5 us).
+    if (grid >= kFillCtas)
+      return launch_vec(top_k == 2 ? combine_vec_kernel<T2, 2, false> : combine_vec_kernel<T2, 0, false>, yy, gates, route_row, oo,
+                        tokens, n_vec, n_vec, top_k, total_rows, 0, s);
+    // Few tokens: the columns are dealt to several CTAs (4 x 4096: 5.5 -> 1.6 us; 600 x 2048, k 4: 5.1 -> 4.5; the same
+    // code with whole rows was 6 % slower at 4096 and 16387 tokens, hence the template).
+    return launch_vec(top_k == 2 ? combine_vec_kernel<T2, 2, true> : combine_vec_kernel<T2, 0, true>, yy, gates, route_row, oo,
                         tokens, n_vec, part_of(n_vec, grid), top_k, total_rows, 0, s);
   } else {
     combine_scalar_kernel<T><<<grid, kWarps * 32, 0, s>>>(static_cast<const T*>(y), gates, route_row,
