@@ -170,7 +170,10 @@ constexpr int kSms = 148;
 constexpr int kMaxSplit = 8;     // CTAs per tile
 constexpr int kMinChunk = 2048;
 
-__global__ void __launch_bounds__(kScatterThreads, 2)
+// (RESIDENT: CTAs per SM that the registers have to leave room for; with the 72 of three, 2049 x 2048 with k = 8, whose
+// tiles rank 256 routes, took 39.7 instead of 34.4 us.)
+template <int RESIDENT>
+__global__ void __launch_bounds__(kScatterThreads, RESIDENT)
 pack_scatter_bulk_kernel(const char* __restrict__ x, const int32_t* __restrict__ idx,
                          const int32_t* __restrict__ tile_hist, const int32_t* __restrict__ tile_base,
                          int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
@@ -347,12 +350,17 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
     // With fewer tiles than half the SMs a tile is copied by up to 8 CTAs; where there are between one and two
     // CTAs per SM the ring is sized for two, so that they run as one wave.  Otherwise a CTA takes a whole tile
     // and the SM's shared memory (a second resident CTA, or a split with 75..148 tiles, was 1..10 % slower).
+    // Up to one and a half tiles per SM a tile is halved, three CTAs per SM: otherwise an SM with two tiles takes twice as
+    // long as the others (device time of the route, k = 2: 4750 x 4096: 42.7 -> 38.8 us, 4750 x 7360: 68.4 -> 62.3,
+    // 7000 x 4096: 47.4 -> 45.0, 5500 x 1024, k 4: 24.7 -> 22.0; 4750 x 512: 13.3 -> 12.8).
     // Device time of the route (router + scatter), before -> after: 16 x 4096, E 64, k 2: 15.7 -> 12.6 us;
     // 600: 21.5 -> 15.1; 1024, E 128, k 4: 34.5 -> 22.5; 2049 x 2048, E 256, k 8: 48.1 -> 41.2;
     // 8192 x 2048, E 32, k 4: 46.2 -> 42.7 us.
     int split = 1;
     if (nt * 2 <= kSms)
       while (split < kMaxSplit && nt * split < kSms) split *= 2;
+    const bool halves = nt > kSms && nt * 2 <= 3 * kSms;
+    if (halves) split = 2;
     const int per_cta = kTileTokens / split;
     int chunk = (int)(row_bytes < (size_t)kChunkBytes ? row_bytes : (size_t)kChunkBytes);
     int chunks = (int)((row_bytes + chunk - 1) / chunk);
@@ -364,7 +372,7 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
     const size_t fixed = (size_t)(2 * experts + 2 * kMaxTileRoutes) * sizeof(int32_t) + 64 * sizeof(uint64_t) + 128;
     const int want = ((per_cta * chunks + kBulkIssuers - 1) / kBulkIssuers) * kBulkIssuers;
     int nbuf = 0;
-    for (int resident = nt * split > kSms && nt * split <= 2 * kSms ? 2 : 1; resident >= 1 && nbuf < kBulkIssuers; --resident)
+    for (int resident = halves ? 3 : nt * split > kSms && nt * split <= 2 * kSms ? 2 : 1; resident >= 1 && nbuf < kBulkIssuers; --resident)
       nbuf = (int)((227 * 1024 / resident - 1024 - fixed) / chunk);
     if (nbuf > want) nbuf = want;
     if (nbuf > 64) nbuf = 64;
@@ -372,12 +380,13 @@ int launch_scan_scatter(const void* x, int elem_bytes, const int32_t* idx, int t
     if (nbuf >= kBulkIssuers) {
       const size_t smem = (size_t)nbuf * chunk + (size_t)nbuf * sizeof(uint64_t) +
                          (size_t)(2 * experts + 2 * kMaxTileRoutes) * sizeof(int32_t);
-      static SmemGrant grant;
-      err = grant_smem(reinterpret_cast<const void*>(pack_scatter_bulk_kernel), smem, grant);
+      static SmemGrant grants[2];
+      const auto kernel = halves ? pack_scatter_bulk_kernel<3> : pack_scatter_bulk_kernel<2>;
+      err = grant_smem(reinterpret_cast<const void*>(kernel), smem, grants[halves]);
       if (err != cudaSuccess) return fail(MOE_ERR_LAUNCH, "pack_scatter_bulk_kernel: %s", cudaGetErrorString(err));
       cfg.gridDim = dim3(nt * split, 1, 1);
       cfg.dynamicSmemBytes = smem;
-      err = cudaLaunchKernelEx(&cfg, pack_scatter_bulk_kernel, xs, idx, th, tile_base, counts, offsets, ps,
+      err = cudaLaunchKernelEx(&cfg, kernel, xs, idx, th, tile_base, counts, offsets, ps,
                                row_route, route_row, tokens, row_bytes, experts, top_k, nt, split, nbuf, chunk,
                                early_rows ? 1 : 0, st, sb);
       if (err != cudaSuccess) return fail(MOE_ERR_LAUNCH, "pack_scatter_bulk_kernel: %s", cudaGetErrorString(err));
