@@ -125,9 +125,6 @@ __device__ __forceinline__ void key_insert(uint32_t (&keys)[KMAX], uint32_t c) {
 }
 
 // ---- cluster-scope mbarrier operations (the exchange of partial tiles) -----------------------------
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
 // Shared memory of this CTA -> shared memory of a CTA of the cluster, completion counted in bytes on an
 // mbarrier of the destination CTA (both given as shared::cluster addresses); 16-byte granularity.
 __device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst_cluster, uint32_t src_cta, uint32_t bytes,
@@ -501,7 +498,7 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
     tc_fence_after();
     if (p.part_in_ring) {
       // the partial tiles that are about to arrive lie where the other CTAs' MMAs have been reading
-      if (ew == 0 && lane < S) mbar_arrive_remote(map_to_cta(part_go, (uint32_t)lane));
+      if (ew == 0 && lane < S) mbar_arrive_cluster(map_to_cta(part_go, (uint32_t)lane));
       mbar_wait_cluster(part_go, 0, p.status, 6);
     }
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
@@ -586,7 +583,7 @@ router_gemm_select_kernel(const __grid_constant__ CUtensorMap tmap_x,
         }
       }
     }
-    if (!p.bulk_push) mbar_arrive_remote(map_to_cta(part_full, (uint32_t)dest));  // releases this thread's stores
+    if (!p.bulk_push) mbar_arrive_cluster(map_to_cta(part_full, (uint32_t)dest));  // releases this thread's stores
     select_phase<KMAX, FORM>(p, s_partial, s_hist, part_full, (kProducers + ew) * 32 + lane, block, krank);
   }
 

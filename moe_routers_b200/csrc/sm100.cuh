@@ -289,7 +289,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Arrive on an mbarrier of the cluster without handing over, at cluster scope, what the thread has written before.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+__device__ __forceinline__ void mbar_arrive_no_release(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
