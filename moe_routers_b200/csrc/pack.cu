@@ -24,6 +24,7 @@ namespace moe {
 namespace {
 
 constexpr int kScatterThreads = 256;
+constexpr long long kEarlySelectBytes = 64LL << 20;
 constexpr int kFusedPrefixTiles = 256;           // up to this many tiles each scatter CTA sums the histograms itself
 
 // ---------------------------------------------------------------------------
@@ -526,7 +527,7 @@ extern "C" int moe_pack_static(const void* x, int elem_bytes, const int32_t* idx
 
 namespace moe {
 int launch_select_any(const void* logits, int logits_dtype, int tokens, int experts, int top_k, int32_t* idx,
-                      float* gates, int32_t* tile_hist, cudaStream_t s);
+                      float* gates, int32_t* tile_hist, cudaStream_t s, bool early);
 }
 
 // The reference's whole operator in two launches: select (+ tile histograms), then scatter.
@@ -549,7 +550,12 @@ extern "C" int moe_fused_select(const void* logits, int logits_dtype, const void
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Workspace ws = carve(workspace, tokens, experts);
   if (tokens > 0) {
-    const int rc = launch_select_any(logits, logits_dtype, tokens, experts, top_k, idx, gates, ws.tile_hist, s);
+    // The select sets itself up under the kernel in front (in a sequence of calls: the last scatter) where the rows take
+    // longer than the host's 15 us for a call: calls of 4096 x 4096: 23.1 -> 22.3 us, 8192 x 2048: 24.7 -> 23.5 (in a graph 22.2
+    // and 23.3 -> 23.6).  Smaller calls took the host longer (1024 x 4096: 15.2 -> 18), and with the scan in between
+    // 12000 x 4096 took 56.2 instead of 53.9 us.
+    const bool early = (1LL + top_k) * tokens * d * elem_bytes >= kEarlySelectBytes && ws.num_tiles <= kFusedPrefixTiles;
+    const int rc = launch_select_any(logits, logits_dtype, tokens, experts, top_k, idx, gates, ws.tile_hist, s, early);
     if (rc != MOE_OK) return rc;
   }
   return launch_scan_scatter(x, elem_bytes, idx, tokens, d, experts, top_k, counts, offsets, packed, row_route,

@@ -131,11 +131,14 @@ __global__ void __launch_bounds__(kFastRows * kFastTpr)
 topk_select16_kernel(const uint16_t* __restrict__ logits, int32_t* __restrict__ out_idx, float* __restrict__ out_w,
                      int tokens, int experts, int top_k, int32_t* __restrict__ tile_hist) {
   extern __shared__ int32_t s_hist[];  // [experts], only with tile_hist
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // a scatter behind us may prefetch its rows
   if (tile_hist != nullptr) {
     for (int e = threadIdx.x; e < experts; e += kFastRows * kFastTpr) s_hist[e] = 0;
     __syncthreads();
   }
+  // May be launched with programmatic stream serialisation: global memory is first touched after the wait, and a scatter
+  // behind us may fetch its rows only then (what is in front may be writing them).
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int row = blockIdx.x * kFastRows + (int)threadIdx.x / kFastTpr;
   const int cg = (int)threadIdx.x % kFastTpr;
   uint32_t keys[KMAX];
@@ -186,18 +189,29 @@ topk_select16_kernel(const uint16_t* __restrict__ logits, int32_t* __restrict__ 
 
 template <bool BF16>
 int launch_select16(const void* logits, int tokens, int experts, int top_k, int32_t* idx, float* w, int32_t* tile_hist,
-                    cudaStream_t s) {
+                    cudaStream_t s, bool early) {
   const uint16_t* p = static_cast<const uint16_t*>(logits);
   const int grid = (tokens + kFastRows - 1) / kFastRows;
   const size_t smem = tile_hist != nullptr ? experts * sizeof(int32_t) : 0;
   const int kmax = top_k <= 1 ? 1 : (top_k <= 2 ? 2 : (top_k <= 4 ? 4 : 8));
-#define MOE_SEL16(K) topk_select16_kernel<K, BF16><<<grid, kFastRows * kFastTpr, smem, s>>>(p, idx, w, tokens, experts, top_k, tile_hist)
-  if (kmax == 1) MOE_SEL16(1);
-  else if (kmax == 2) MOE_SEL16(2);
-  else if (kmax == 4) MOE_SEL16(4);
-  else MOE_SEL16(8);
-#undef MOE_SEL16
-  return check_launch("topk_select16_kernel");
+  const auto kernel = kmax == 1   ? topk_select16_kernel<1, BF16>
+                      : kmax == 2 ? topk_select16_kernel<2, BF16>
+                      : kmax == 4 ? topk_select16_kernel<4, BF16>
+                                  : topk_select16_kernel<8, BF16>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(kFastRows * kFastTpr, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early && pdl_enabled() ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, idx, w, tokens, experts, top_k, tile_hist);
+  if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "topk_select16_kernel: %s", cudaGetErrorString(e));
+  note_launch();
+  return MOE_OK;
 }
 
 template <typename T>
@@ -226,14 +240,15 @@ int launch_select(const void* logits, int tokens, int experts, int top_k, int32_
 
 }  // namespace
 
-// select (+ per-tile histogram when tile_hist is given) for any logits dtype
+// select (+ per-tile histogram when tile_hist is given) for any logits dtype; `early`: it may set itself up under the
+// kernel in front
 int launch_select_any(const void* logits, int logits_dtype, int tokens, int experts, int top_k, int32_t* idx,
-                      float* gates, int32_t* tile_hist, cudaStream_t s) {
+                      float* gates, int32_t* tile_hist, cudaStream_t s, bool early) {
   // 16-bit logits with 16-byte rows: the key-based kernel (every pick of a row must exist: top_k <= experts)
   if ((logits_dtype == MOE_F16 || logits_dtype == MOE_BF16) && experts % 8 == 0 && experts <= 1024 &&
       (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
-    return logits_dtype == MOE_F16 ? launch_select16<false>(logits, tokens, experts, top_k, idx, gates, tile_hist, s)
-                                   : launch_select16<true>(logits, tokens, experts, top_k, idx, gates, tile_hist, s);
+    return logits_dtype == MOE_F16 ? launch_select16<false>(logits, tokens, experts, top_k, idx, gates, tile_hist, s, early)
+                                   : launch_select16<true>(logits, tokens, experts, top_k, idx, gates, tile_hist, s, early);
   }
   switch (logits_dtype) {
     case MOE_F16: return launch_select<__half>(logits, tokens, experts, top_k, idx, gates, tile_hist, s);
@@ -255,5 +270,5 @@ extern "C" int moe_topk_select(const void* logits, int logits_dtype, int tokens,
   if (tokens == 0) return MOE_OK;
   if (!logits || !idx || !gates) return fail(MOE_ERR_ARG, "moe_topk_select: null pointer");
   return launch_select_any(logits, logits_dtype, tokens, experts, top_k, idx, gates, nullptr,
-                           static_cast<cudaStream_t>(stream));
+                           static_cast<cudaStream_t>(stream), false);
 }
