@@ -406,10 +406,11 @@ PyObject* expert_ffn(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // The tensors of a list as one buffer: all fp16, of `cols` columns (and, with `same_rows`, of one shape), each
-// beginning where the one before it ends, inside one storage.  Tensors without rows lie anywhere.
-bool one_buffer(PyObject* list, long dev, int64_t cols, bool same_rows, const at::Tensor*& first, int64_t& rows, int64_t* counts) {
+// beginning where the one before it ends, inside one storage.  Tensors without rows lie anywhere.  `first` becomes a
+// reference of its own, which holds that storage: the list is the caller's, and another thread may change it as soon as
+// the GIL is given up or Python code runs.
+bool one_buffer(PyObject* list, long dev, int64_t cols, bool same_rows, at::Tensor& first, int64_t& rows, int64_t* counts) {
   const Py_ssize_t n = PyList_GET_SIZE(list);
-  first = nullptr;
   rows = 0;
   const char* next = nullptr;
   for (Py_ssize_t i = 0; i < n; ++i) {
@@ -420,12 +421,12 @@ bool one_buffer(PyObject* list, long dev, int64_t cols, bool same_rows, const at
     if (same_rows && counts[i] != counts[0]) return false;
     if (t->numel() == 0) continue;
     const char* at = static_cast<const char*>(t->data_ptr());
-    if (first == nullptr) first = t;
+    if (!first.defined()) first = *t;
     else if (at != next) return false;
     next = at + t->numel() * 2;
   }
-  if (first == nullptr || rows > kMaxInt) return false;
-  const c10::Storage& storage = first->storage();
+  if (!first.defined() || rows > kMaxInt) return false;
+  const c10::Storage& storage = first.storage();
   return next <= static_cast<const char*>(storage.data()) + storage.nbytes();
 }
 
@@ -439,7 +440,7 @@ PyObject* grouped_lists(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const at::Tensor* w0 = plain(PyList_GET_ITEM(args[3], 0), c.dev, 2);
   if (!w0) Py_RETURN_NONE;
   const int64_t k = w0->size(0), cols = w0->size(1);
-  const at::Tensor *a, *w;
+  at::Tensor a, w;
   int64_t rows, w_rows;
   c10::SmallVector<int64_t, 64> counts(e), w_counts(e);
   if (k > kMaxInt || cols > kMaxInt || !one_buffer(args[2], c.dev, k, false, a, rows, counts.data()) ||
@@ -455,7 +456,7 @@ PyObject* grouped_lists(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const at::Tensor offsets = c.make({e + 1}, at::kInt), out = c.make({rows, cols}, at::kHalf);
     rc = api.store_offsets(ends.data(), (int)e + 1, data<int32_t>(offsets), c.stream);
     if (rc == MOE_OK)
-      rc = api.grouped_gemm(a->data_ptr(), w->data_ptr(), out.data_ptr(), data<int32_t>(offsets), (int)e, (int)rows, (int)k, (int)cols,
+      rc = api.grouped_gemm(a.data_ptr(), w.data_ptr(), out.data_ptr(), data<int32_t>(offsets), (int)e, (int)rows, (int)k, (int)cols,
                             MOE_W_KN, k * cols, MOE_ACT_NONE, nullptr, nullptr, MOE_F16, 0, c.ws, c.ws_bytes, c.stream);
     if (rc == MOE_OK) pieces = out.split_with_sizes(counts, 0);
   }

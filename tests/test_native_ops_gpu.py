@@ -87,6 +87,29 @@ def test_grouped_lists(counts):
 
 
 @pytest.mark.gpu
+def test_grouped_lists_holds_its_buffers(monkeypatch):
+    """Whoever empties the lists during the call (here the code that makes the scratch buffer, in a program another thread)
+    does not take the rows and weights away from it."""
+    from moe_routers_b200 import ops
+
+    a, w = _randn(12, 64), _randn(4, 64, 64, seed=1) / 8
+    want = torch.cat(ops.grouped_lists(list(a.clone().split(3)), list(w.clone().unbind(0))))
+    ins, ws, spoiled, stream = list(a.clone().split(3)), list(w.clone().unbind(0)), [], ops._stream
+
+    def meanwhile():
+        ins.clear(), ws.clear()
+        spoiled.extend(torch.full_like(t, float("nan")) for t in (a, w) for _ in range(4))  # what was given back is taken
+        return stream()
+
+    ops._workspaces.pop((torch.cuda.current_device(), stream()), None)
+    monkeypatch.setattr(ops, "_stream", meanwhile)
+    out = ops.grouped_lists(ins, ws)
+    monkeypatch.undo()
+    assert spoiled
+    _same(torch.cat(out), want)
+
+
+@pytest.mark.gpu
 def test_errors_are_those_of_the_general_path():
     from moe_routers_b200 import ops
     from moe_routers_b200._lib import MoeError
