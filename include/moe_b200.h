@@ -227,7 +227,7 @@ int moe_dense_experts(const void* a, const void* w, void* c, int experts, int to
  * The gate-masked sum behind it: out[t] = sum_e g[t,e] * y[e * tokens + t], g[t,e] the gate of t's pick of e, 0 where
  * e was not picked (the row is read and multiplied all the same), accumulated in fp32 in ascending e.
  *   y [experts * tokens, d] fp16/bf16, idx [tokens, top_k] int32, gates [tokens, top_k] float32, out [tokens, d]
- * Limits: experts <= 8, top_k <= 8, d a multiple of 8, y and out 16-byte aligned.
+ * Limits: experts <= 8, top_k <= 8, d a multiple of 8, y and out 16-byte aligned, experts * tokens < 2^31.
  */
 int moe_combine_dense(const void* y, int dtype, const int32_t* idx, const float* gates, int tokens, int d, int experts,
                       int top_k, void* out, void* stream);

@@ -218,6 +218,7 @@ extern "C" int moe_combine_dense(const void* y, int dtype, const int32_t* idx, c
   if (tokens < 0 || d <= 0 || d % 8 != 0) return fail(MOE_ERR_ARG, "moe_combine_dense: bad shape");
   if (experts < 1 || experts > 8) return fail(MOE_ERR_UNSUPPORTED, "moe_combine_dense: experts must be in [1,8], got %d", experts);
   if (top_k < 1 || top_k > 8) return fail(MOE_ERR_UNSUPPORTED, "moe_combine_dense: top_k must be in [1,8], got %d", top_k);
+  if ((long long)experts * tokens > 0x7fffffffLL) return fail(MOE_ERR_UNSUPPORTED, "moe_combine_dense: too many rows");
   if (tokens == 0) return MOE_OK;
   if (!y || !idx || !gates || !out) return fail(MOE_ERR_ARG, "moe_combine_dense: null pointer");
   if ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15)

@@ -88,6 +88,10 @@ def test_argument_errors_do_not_launch(lib):
     assert 0 <= before <= 31
     assert L.moe_set_gemm_mode(5) == before and L.moe_set_gemm_mode(-1) == 5
     assert L.moe_set_gemm_mode(before) == 5 and L.moe_set_gemm_mode(-1) == before
+    # the kernels index the rows of all experts with 32 bits
+    some = ctypes.c_void_p(4096)
+    rc = L.moe_combine_dense(some, lib.MOE_F16, some, some, 300_000_000, 8, 8, 2, some, None)
+    assert rc == 2 and "too many rows" in lib.last_error()
     # zero tokens is a valid no-op that needs no pointers
     assert L.moe_topk_select(None, lib.MOE_F16, 0, 64, 2, None, None, None) == 0
     assert L.moe_combine(None, lib.MOE_F16, None, None, 0, 8, 2, None, None) == 0
