@@ -20,6 +20,8 @@ from ._lib import check, lib
 
 _DTYPE_CODE = {torch.float16: _lib.MOE_F16, torch.bfloat16: _lib.MOE_BF16, torch.float32: _lib.MOE_F32}
 
+_MAX_ROWS = 2 ** 31 - 1  # what the library's int arguments hold
+
 _workspaces: dict = {}
 
 
@@ -427,10 +429,14 @@ def combine_dense(y: torch.Tensor, idx: torch.Tensor, gates: torch.Tensor, exper
     _require_cuda(y, idx, gates)
     if y.dtype not in (torch.float16, torch.bfloat16):
         raise RuntimeError("y must be fp16 or bf16")
+    if y.dim() != 2 or idx.dim() != 2 or idx.shape != gates.shape or y.size(0) != experts * idx.size(0):
+        raise RuntimeError("combine_dense: expected y [experts * T, d] and idx, gates [T, top_k]")
+    if y.size(0) > _MAX_ROWS:
+        raise RuntimeError("combine_dense: too many rows")
     y = y.contiguous()
     idx = idx.to(torch.int32).contiguous()
     gates = gates.to(torch.float32).contiguous()
-    t, d = y.size(0) // experts, y.size(1)
+    t, d = idx.size(0), y.size(1)
     dev = y.get_device()
     with _on(dev):
         out, = empties(dev, ((y.dtype, t, d),))

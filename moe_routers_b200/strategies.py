@@ -59,7 +59,14 @@ def masked_matmul_forward(x: torch.Tensor, r: dict, w1: torch.Tensor, w2: torch.
         e1 = min(e, e0 + at_once)
         h = ops.dense_experts(x, w1[e0:e1], t, activation=activation)
         ops.dense_experts(h, w2[e0:e1], t, out=y[e0 * t:e1 * t])
-    return ops.combine_dense(y, r["idx"], r["gates"], e)
+    idx, gates = r["idx"], r["gates"]
+    if not (idx.dim() == 2 and idx.shape == gates.shape and idx.size(0) == t and 1 <= idx.size(1) <= 8
+            and idx.device == gates.device == x.device):
+        # a routing of fewer tokens (the others get nothing), gates wider than the picks, more picks than the kernel takes:
+        # as a mask over all experts, which raises where the shapes or devices do not go together
+        mask = torch.zeros((t, e), dtype=torch.float32, device=x.device).scatter_add_(1, idx.long(), gates)
+        idx, gates = torch.arange(e, dtype=torch.int32, device=x.device).expand(t, e), mask
+    return ops.combine_dense(y, idx, gates, e)
 
 
 _HIDDEN_BYTES = 512 << 20  # of masked_matmul_forward's hidden rows
