@@ -228,9 +228,13 @@ int moe_dense_experts(const void* a, const void* w, void* c, int experts, int to
  * e was not picked (the row is read and multiplied all the same), accumulated in fp32 in ascending e.
  *   y [experts * tokens, d] fp16/bf16, idx [tokens, top_k] int32, gates [tokens, top_k] float32, out [tokens, d]
  * Limits: experts <= 8, top_k <= 8, d a multiple of 8, y and out 16-byte aligned, experts * tokens < 2^31.
+ * A pick outside [0, experts) adds nothing; the second form records it in `device_status` (the first word of a
+ * workspace, see moe_read_status; may be null).
  */
 int moe_combine_dense(const void* y, int dtype, const int32_t* idx, const float* gates, int tokens, int d, int experts,
                       int top_k, void* out, void* stream);
+int moe_combine_dense_checked(const void* y, int dtype, const int32_t* idx, const float* gates, int tokens, int d,
+                              int experts, int top_k, void* out, int32_t* device_status, void* stream);
 
 /*
  * Gate-weighted un-permute and sum over the top_k picks:

@@ -58,6 +58,7 @@ SIGNATURES = {
     "moe_expert_ffn": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _p, _i, _p, _i, _p, _sz, _p]),
     "moe_dense_experts": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, C.c_int64, _i, _i, _p, _sz, _p]),
     "moe_combine_dense": (_i, [_p, _i, _p, _p, _i, _i, _i, _i, _p, _p]),
+    "moe_combine_dense_checked": (_i, [_p, _i, _p, _p, _i, _i, _i, _i, _p, _p, _p]),
     "moe_pack_scatter_to": (_i, [_p, _i, _p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p, _sz, _p]),
     "moe_ep_segment_bases": (_i, [_p, _p, _i, _i, _i, _i, _i, _p, _p, _p]),
     "moe_ep_row_targets": (_i, [_p, _p, _i, _i, _i, _i, _i, _p, _p]),

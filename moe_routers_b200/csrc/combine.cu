@@ -38,12 +38,12 @@ __device__ __forceinline__ uint32_t pack2<__nv_bfloat162>(float a, float b) {
 
 // Vector path: d % 8 == 0 and 16-byte aligned bases.  DENSE: the rows are those of all experts (`top_k_rt` of them,
 // expert e's row of token t at e * tokens + t), `route_row` holds the token's `picks` experts, and a row's gate is
-// that of the pick of its expert, or 0.
+// that of the pick of its expert, or 0.  A pick of an expert that does not exist counts nowhere and is recorded in `status`.
 template <typename T2, int TOPK, bool SPLIT, bool DENSE = false>
 __global__ void __launch_bounds__(kWarps * 32)
 combine_vec_kernel(const uint4* __restrict__ y, const float* __restrict__ gates,
                    const int32_t* __restrict__ route_row, uint4* __restrict__ out, int tokens,
-                   int n_vec_total, int part_vec, int top_k_rt, int total_rows, int picks = 0) {
+                   int n_vec_total, int part_vec, int top_k_rt, int total_rows, int picks = 0, int32_t* status = nullptr) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * kWarps + (threadIdx.x >> 5);
   // launched with programmatic stream serialisation: everything in global memory is touched after this
@@ -55,6 +55,9 @@ combine_vec_kernel(const uint4* __restrict__ y, const float* __restrict__ gates,
   const int v_begin = SPLIT ? blockIdx.y * part_vec : 0;  // this warp's 16-byte pieces of the row
   const int n_vec = SPLIT ? min(n_vec_total, v_begin + part_vec) : n_vec_total;
   const int top_k = TOPK > 0 ? TOPK : top_k_rt;
+  if constexpr (DENSE) {
+    if (lane < picks && (unsigned)__ldg(route_row + (size_t)t * picks + lane) >= (unsigned)top_k) record_error(status, kErrBadIndex);
+  }
   const uint4* src[8];
   float g[8];
 #pragma unroll
@@ -145,7 +148,7 @@ inline int part_of(int n_vec, int grid) {
 }
 template <typename Kernel>
 int launch_vec(Kernel kernel, const uint4* y, const float* gates, const int32_t* rows, uint4* out, int tokens, int n_vec,
-                 int part, int top_k, int total_rows, int picks, cudaStream_t s) {
+                 int part, int top_k, int total_rows, int picks, int32_t* status, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((tokens + kWarps - 1) / kWarps, (n_vec + part - 1) / part, 1);
   cfg.blockDim = dim3(kWarps * 32, 1, 1);
@@ -155,7 +158,7 @@ int launch_vec(Kernel kernel, const uint4* y, const float* gates, const int32_t*
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, y, gates, rows, out, tokens, n_vec, part, top_k, total_rows, picks);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, y, gates, rows, out, tokens, n_vec, part, top_k, total_rows, picks, status);
   if (e != cudaSuccess) return fail(MOE_ERR_LAUNCH, "combine_kernel: %s", cudaGetErrorString(e));
   note_launch();
   return MOE_OK;
@@ -163,10 +166,10 @@ int launch_vec(Kernel kernel, const uint4* y, const float* gates, const int32_t*
 
 template <typename T2>
 int launch_combine_dense(const void* y, const int32_t* idx, const float* gates, int tokens, int d, int experts, int top_k,
-                         void* out, cudaStream_t s) {
+                         void* out, int32_t* status, cudaStream_t s) {
   const int n_vec = d / 8;
   return launch_vec(combine_vec_kernel<T2, 0, true, true>, static_cast<const uint4*>(y), gates, idx, static_cast<uint4*>(out),
-                      tokens, n_vec, part_of(n_vec, (tokens + kWarps - 1) / kWarps), experts, experts * tokens, top_k, s);
+                      tokens, n_vec, part_of(n_vec, (tokens + kWarps - 1) / kWarps), experts, experts * tokens, top_k, status, s);
 }
 
 template <typename T, typename T2>
@@ -182,11 +185,11 @@ int launch_combine(const void* y, const float* gates, const int32_t* route_row, 
     // Set up under the GEMM in front of it in either form (layer of 3330 x 768: 67.5 -> 65.5 us).
     if (grid >= kFillCtas)
       return launch_vec(top_k == 2 ? combine_vec_kernel<T2, 2, false> : combine_vec_kernel<T2, 0, false>, yy, gates, route_row, oo,
-                        tokens, n_vec, n_vec, top_k, total_rows, 0, s);
+                        tokens, n_vec, n_vec, top_k, total_rows, 0, nullptr, s);
     // Few tokens: the columns are dealt to several CTAs (4 x 4096: 5.5 -> 1.6 us; 600 x 2048, k 4: 5.1 -> 4.5; the same
     // code with whole rows was 6 % slower at 4096 and 16387 tokens, hence the template).
     return launch_vec(top_k == 2 ? combine_vec_kernel<T2, 2, true> : combine_vec_kernel<T2, 0, true>, yy, gates, route_row, oo,
-                        tokens, n_vec, part_of(n_vec, grid), top_k, total_rows, 0, s);
+                        tokens, n_vec, part_of(n_vec, grid), top_k, total_rows, 0, nullptr, s);
   } else {
     combine_scalar_kernel<T><<<grid, kWarps * 32, 0, s>>>(static_cast<const T*>(y), gates, route_row,
                                                          static_cast<T*>(out), tokens, d, top_k, total_rows);
@@ -212,8 +215,8 @@ extern "C" int moe_combine(const void* y, int dtype, const float* gates, const i
   }
 }
 
-extern "C" int moe_combine_dense(const void* y, int dtype, const int32_t* idx, const float* gates, int tokens, int d,
-                                 int experts, int top_k, void* out, void* stream) {
+extern "C" int moe_combine_dense_checked(const void* y, int dtype, const int32_t* idx, const float* gates, int tokens, int d,
+                                         int experts, int top_k, void* out, int32_t* device_status, void* stream) {
   using namespace moe;
   if (tokens < 0 || d <= 0 || d % 8 != 0) return fail(MOE_ERR_ARG, "moe_combine_dense: bad shape");
   if (experts < 1 || experts > 8) return fail(MOE_ERR_UNSUPPORTED, "moe_combine_dense: experts must be in [1,8], got %d", experts);
@@ -225,8 +228,13 @@ extern "C" int moe_combine_dense(const void* y, int dtype, const int32_t* idx, c
     return fail(MOE_ERR_ARG, "moe_combine_dense: y and out must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (dtype) {
-    case MOE_F16: return launch_combine_dense<__half2>(y, idx, gates, tokens, d, experts, top_k, out, s);
-    case MOE_BF16: return launch_combine_dense<__nv_bfloat162>(y, idx, gates, tokens, d, experts, top_k, out, s);
+    case MOE_F16: return launch_combine_dense<__half2>(y, idx, gates, tokens, d, experts, top_k, out, device_status, s);
+    case MOE_BF16: return launch_combine_dense<__nv_bfloat162>(y, idx, gates, tokens, d, experts, top_k, out, device_status, s);
     default: return fail(MOE_ERR_ARG, "moe_combine_dense: dtype must be fp16 or bf16");
   }
+}
+
+extern "C" int moe_combine_dense(const void* y, int dtype, const int32_t* idx, const float* gates, int tokens, int d,
+                                 int experts, int top_k, void* out, void* stream) {
+  return moe_combine_dense_checked(y, dtype, idx, gates, tokens, d, experts, top_k, out, nullptr, stream);
 }

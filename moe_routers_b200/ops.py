@@ -425,7 +425,8 @@ def dense_experts(a: torch.Tensor, w: torch.Tensor, tokens: int, *, activation: 
 
 
 def combine_dense(y: torch.Tensor, idx: torch.Tensor, gates: torch.Tensor, experts: int) -> torch.Tensor:
-    """out[t] = sum_e g[t, e] * y[e * T + t] with the gate of t's pick of expert e, 0 for the experts not picked."""
+    """out[t] = sum_e g[t, e] * y[e * T + t] with the gate of t's pick of expert e, 0 for the experts not picked.
+    A pick outside [0, E) adds nothing and is reported by `read_status`."""
     _require_cuda(y, idx, gates)
     if y.dtype not in (torch.float16, torch.bfloat16):
         raise RuntimeError("y must be fp16 or bf16")
@@ -440,8 +441,9 @@ def combine_dense(y: torch.Tensor, idx: torch.Tensor, gates: torch.Tensor, exper
     dev = y.get_device()
     with _on(dev):
         out, = empties(dev, ((y.dtype, t, d),))
-        check(lib.moe_combine_dense(y.data_ptr(), _DTYPE_CODE[y.dtype], idx.data_ptr(), gates.data_ptr(), t, d, int(experts),
-                                    idx.size(1), out.data_ptr(), _stream()))
+        check(lib.moe_combine_dense_checked(y.data_ptr(), _DTYPE_CODE[y.dtype], idx.data_ptr(), gates.data_ptr(), t, d,
+                                            int(experts), idx.size(1), out.data_ptr(), _workspace(dev, 1, 1, 1).data_ptr(),
+                                            _stream()))
     return out
 
 

@@ -49,3 +49,23 @@ def test_infinite_rows_of_experts_not_picked_still_count():
     idx = torch.zeros(16, 1, dtype=torch.int32, device="cuda")
     out = ops.combine_dense(y, idx, torch.ones(16, 1, device="cuda"), 2)
     assert torch.isnan(out[3]).all() and (out[torch.arange(16) != 3] == 1).all()
+
+
+@pytest.mark.parametrize("bad", [-1, 4, 1 << 30])
+def test_picks_of_experts_that_do_not_exist_are_reported(bad):
+    """They add nothing, and the status of the stream says so."""
+    from moe_routers_b200 import ops
+    from moe_routers_b200._lib import MoeError
+
+    y = torch.ones(4 * 40, 8, dtype=torch.bfloat16, device="cuda")
+    idx = torch.tensor([[0, 3]], dtype=torch.int32, device="cuda").repeat(40, 1)
+    gates = torch.tensor([[1.0, 2.0]], device="cuda").repeat(40, 1)
+    assert (ops.combine_dense(y, idx, gates, 4) == 3).all() and ops.read_status() == 0
+    idx[37, 1] = bad
+    try:
+        out = ops.combine_dense(y, idx, gates, 4)
+        assert (out[37] == 1).all() and (out[torch.arange(40) != 37] == 3).all()
+        with pytest.raises(MoeError, match="expert index"):
+            ops.read_status()
+    finally:  # the status block again as the other tests expect it
+        ops.workspace(torch.device("cuda"), 1, 1, 1)[:4].zero_()
