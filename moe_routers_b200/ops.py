@@ -403,8 +403,8 @@ def dense_experts(a: torch.Tensor, w: torch.Tensor, tokens: int, *, activation: 
     _require_cuda(a, w)
     if a.dtype not in (torch.float16, torch.bfloat16) or w.dtype != a.dtype:
         raise RuntimeError("grouped_gemm: a and w must both be fp16 or both bf16")
-    if w.dim() != 3:
-        raise RuntimeError("grouped_gemm: w must be [E, N, K]")
+    if a.dim() != 2 or w.dim() != 3:
+        raise RuntimeError("dense_experts: expected a [rows, K] and w [E, N, K]")
     a = a.contiguous()
     w = w.contiguous()
     e, n_w, k_dim = w.shape
@@ -412,8 +412,13 @@ def dense_experts(a: torch.Tensor, w: torch.Tensor, tokens: int, *, activation: 
         raise RuntimeError("grouped_gemm: inner dimensions differ")
     if a.size(0) not in (tokens, e * tokens):
         raise RuntimeError("dense_experts: a must have tokens or experts * tokens rows")
+    if e * tokens > _MAX_ROWS:
+        raise RuntimeError("dense_experts: too many rows")
     act = _ACT[activation]
     n_out = n_w // 2 if act == _lib.MOE_ACT_SWIGLU else n_w
+    if out is not None and (out.shape != (e * tokens, n_out) or out.dtype != a.dtype or out.device != a.device
+                            or not out.is_contiguous()):
+        raise RuntimeError(f"dense_experts: out must be a contiguous [{e * tokens}, {n_out}] tensor like a")
     dev = a.get_device()
     with _on(dev):
         ws = _workspace(dev, 1, e, 1)

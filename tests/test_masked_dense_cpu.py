@@ -72,3 +72,13 @@ def test_combine_dense_refuses_shapes_that_do_not_belong_together(no_gpu, rows, 
     with pytest.raises(RuntimeError, match="combine_dense: expected"):
         ops.combine_dense(torch.zeros(rows, 8, dtype=torch.float16), torch.zeros(idx_shape, dtype=torch.int32),
                           torch.zeros(gates_shape), 4)
+
+
+@pytest.mark.parametrize("out", [
+    torch.empty(31, 24, dtype=torch.float16), torch.empty(32, 16, dtype=torch.float16), torch.empty(32, 32, dtype=torch.float16),
+    torch.empty(32, 24, dtype=torch.bfloat16), torch.empty(32, 48, dtype=torch.float16)[:, ::2], torch.empty(768, dtype=torch.float16),
+    torch.empty(32, 24, dtype=torch.float16, device="meta")])
+def test_dense_experts_refuses_an_output_that_is_not_its_own(no_gpu, out):
+    a, w = torch.zeros(8, 16, dtype=torch.float16), torch.zeros(4, 24, 16, dtype=torch.float16)
+    with pytest.raises(RuntimeError, match="out must be"):
+        ops.dense_experts(a, w, 8, out=out)
