@@ -277,7 +277,7 @@ PyObject* route(PyObject*, PyObject* const* args, Py_ssize_t n) {
       !small_int(args[4], 1, 8, k) || !small_int(args[5], -kMaxInt, kMaxInt, skew) || !number(args[6], bias)) Py_RETURN_NONE;
   const bool with_logits = args[7] == Py_True;
   const int64_t t = x->size(0), d = x->size(1), e = w->size(0);
-  if (e == 0 || t * k > kMaxInt) Py_RETURN_NONE;
+  if (e == 0 || w->size(1) != d || t * k > kMaxInt) Py_RETURN_NONE;
   c.workspace(args[0], (int)t, (int)e, k);
   Routing r;
   int rc;

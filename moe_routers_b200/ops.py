@@ -236,12 +236,18 @@ def combine(y: torch.Tensor, gates: torch.Tensor, route_row: torch.Tensor, top_k
     return out
 
 
+def _check_router_weight(x: torch.Tensor, w_router: torch.Tensor) -> None:
+    if w_router.dim() != 2 or x.dim() != 2 or w_router.size(1) != x.size(1):
+        raise RuntimeError("x must be [T, d_model] and the router weight must be [n_experts, d_model]")
+
+
 def router_gemm_select(x: torch.Tensor, w_router: torch.Tensor, top_k: int, *, skew_experts: int = 0,
                        skew_bias: float = 0.0, return_logits: bool = False):
     """Fused logit GEMM + skew + top-k + gates.  Returns (idx, gates[, logits fp32])."""
     _require_cuda(x, w_router)
     if x.dtype not in (torch.float16, torch.bfloat16) or w_router.dtype != x.dtype:
         raise RuntimeError("x and the router weight must both be fp16 (Half) or both bf16")
+    _check_router_weight(x, w_router)
     x = x.contiguous()
     w_router = w_router.contiguous()
     t, d = x.shape
@@ -276,6 +282,7 @@ def route_fused(x: torch.Tensor, w_router: torch.Tensor, top_k: int, *, skew_exp
     _require_cuda(x, w_router)
     if x.dtype not in (torch.float16, torch.bfloat16) or w_router.dtype != x.dtype:
         raise RuntimeError("x and the router weight must both be fp16 (Half) or both bf16")
+    _check_router_weight(x, w_router)
     x = x.contiguous()
     w_router = w_router.contiguous()
     t, d = x.shape

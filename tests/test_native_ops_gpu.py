@@ -119,6 +119,8 @@ def test_errors_are_those_of_the_general_path():
         ops.route_fused(x, w, 9)
     with pytest.raises(RuntimeError, match="fp16"):
         ops.route_fused(x, w.float(), 2)
+    with pytest.raises(RuntimeError, match="router weight must be"):
+        ops.route_fused(x, _randn(8, 56), 2)
     with pytest.raises(MoeError, match="epsilon"):
         ops.sinkhorn(x, 2, epsilon=0.0)
     with pytest.raises(MoeError, match="n_experts"):
