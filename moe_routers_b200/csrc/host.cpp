@@ -328,7 +328,7 @@ PyObject* fused_select(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (!logits || !x || type_code(*logits) < 0 || !fits(*x) || x->element_size() > kMaxInt || !small_int(args[4], 1, 1024, e) ||
       !small_int(args[5], 1, 8, k)) Py_RETURN_NONE;
   const int64_t t = x->size(0), d = x->size(1);
-  if (t * k > kMaxInt) Py_RETURN_NONE;
+  if (logits->size(0) < t || logits->size(1) != e || t * k > kMaxInt) Py_RETURN_NONE;
   c.workspace(args[0], (int)t, e, k);
   Routing r;
   int rc;

@@ -200,9 +200,11 @@ def fused_select(logits: torch.Tensor, x: torch.Tensor, experts: int, top_k: int
     _require_cuda(logits, x)
     if logits.dtype not in _DTYPE_CODE:
         raise RuntimeError("logits must be fp16/bf16/fp32")
+    t, d = x.shape
+    if logits.numel() < t * experts or (logits.dim() > 1 and logits.size(-1) != experts):
+        raise RuntimeError("logits must be [T, n_experts] for x [T, d_model]")
     logits = logits.contiguous()
     x = x.contiguous()
-    t, d = x.shape
     dev = x.get_device()
     with _on(dev):
         if out is None:

@@ -125,6 +125,11 @@ def test_errors_are_those_of_the_general_path():
         ops.sinkhorn(x, 2, epsilon=0.0)
     with pytest.raises(MoeError, match="n_experts"):
         ops.fused_select(_randn(4, 4), x, 4, 8)
+    for logits in (_randn(3, 8), _randn(4, 7)):
+        with pytest.raises(RuntimeError, match="logits must be"):
+            ops.fused_select(logits, x, 8, 2)
+    for a, b in zip(ops.fused_select(torch.cat([w[:, :8], w[:, 8:16]])[:9], x, 8, 2), ops.fused_select(w[:4, :8], x, 8, 2)):
+        _same(a, b)  # more logits than tokens: the first ones, as ever
     with pytest.raises(RuntimeError, match="inner dimensions"):
         o = ops.route_fused(x, w, 2)
         ops.expert_ffn(o["packed"], _randn(8, 64, 32), w.view(8, 8, 8), o["offsets"], o["gates"], o["route_row"], 2, activation=None)

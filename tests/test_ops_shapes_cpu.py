@@ -20,3 +20,9 @@ def _half(*shape):
 def test_router_weight_of_another_width(route, w):
     with pytest.raises(RuntimeError, match="router weight must be"):
         route(_half(4, 64), w, 2)
+
+
+@pytest.mark.parametrize("logits", [_half(3, 8), _half(4, 7), _half(4, 16), _half(31), _half(2, 1, 8)])
+def test_logits_of_another_shape(logits):
+    with pytest.raises(RuntimeError, match="logits must be"):
+        ops.fused_select(logits, _half(4, 64), 8, 2)
