@@ -201,7 +201,7 @@ def fused_select(logits: torch.Tensor, x: torch.Tensor, experts: int, top_k: int
     if logits.dtype not in _DTYPE_CODE:
         raise RuntimeError("logits must be fp16/bf16/fp32")
     t, d = x.shape
-    if logits.numel() < t * experts or (logits.dim() > 1 and logits.size(-1) != experts):
+    if logits.numel() < t * experts or (logits.numel() > t * experts and logits.dim() > 1 and logits.size(-1) != experts):
         raise RuntimeError("logits must be [T, n_experts] for x [T, d_model]")
     logits = logits.contiguous()
     x = x.contiguous()

@@ -128,6 +128,8 @@ def test_errors_are_those_of_the_general_path():
     for logits in (_randn(3, 8), _randn(4, 7)):
         with pytest.raises(RuntimeError, match="logits must be"):
             ops.fused_select(logits, x, 8, 2)
+    for a, b in zip(ops.fused_select(w.view(4, 128)[:, :8].reshape(2, 16), x, 8, 2), ops.fused_select(w[::2, :8], x, 8, 2)):
+        _same(a, b)  # as many in another shape: row by row
     for a, b in zip(ops.fused_select(torch.cat([w[:, :8], w[:, 8:16]])[:9], x, 8, 2), ops.fused_select(w[:4, :8], x, 8, 2)):
         _same(a, b)  # more logits than tokens: the first ones, as ever
     with pytest.raises(RuntimeError, match="inner dimensions"):
