@@ -230,6 +230,10 @@ def combine(y: torch.Tensor, gates: torch.Tensor, route_row: torch.Tensor, top_k
     route_row = route_row.to(torch.int32).contiguous()
     rows, d = y.shape
     t = rows // top_k
+    if gates.numel() < t * top_k or (gates.numel() > t * top_k and gates.dim() > 1 and gates.size(-1) != top_k):
+        raise RuntimeError("combine: gates must be [T, top_k] for y [T * top_k, d]")
+    if route_row.numel() < t * top_k:
+        raise RuntimeError("combine: route_row must have one row per route")
     dev = y.get_device()
     with _on(dev):
         out, = empties(dev, ((y.dtype, t, d),))
@@ -378,6 +382,8 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, *, lay
     n_w = w.size(1) if layout == "nk" else w.size(2)
     if (w.size(2) if layout == "nk" else w.size(1)) != k_dim:
         raise RuntimeError("grouped_gemm: inner dimensions differ")
+    if offsets.numel() <= e:
+        raise RuntimeError("grouped_gemm: offsets must have experts + 1 entries")
     act = _ACT[activation]
     n_out = n_w // 2 if act == _lib.MOE_ACT_SWIGLU else n_w
     dev = a.get_device()

@@ -132,6 +132,11 @@ def test_errors_are_those_of_the_general_path():
         _same(a, b)  # as many in another shape: row by row
     for a, b in zip(ops.fused_select(torch.cat([w[:, :8], w[:, 8:16]])[:9], x, 8, 2), ops.fused_select(w[:4, :8], x, 8, 2)):
         _same(a, b)  # more logits than tokens: the first ones, as ever
+    o = ops.route_fused(x, w, 2)
+    for name, short, text in (("offsets", o["offsets"][:8], "offsets must have"), ("gates", o["gates"][:3], "gates must be"),
+                              ("gates", o["gates"].repeat(1, 2), "gates must be"), ("route_row", o["route_row"][:7], "route_row must")):
+        r = {**o, name: short}
+        with pytest.raises(RuntimeError, match=text):
+            ops.expert_ffn(r["packed"], _randn(8, 64, 64), _randn(8, 64, 64), r["offsets"], r["gates"], r["route_row"], 2, activation=None)
     with pytest.raises(RuntimeError, match="inner dimensions"):
-        o = ops.route_fused(x, w, 2)
         ops.expert_ffn(o["packed"], _randn(8, 64, 32), w.view(8, 8, 8), o["offsets"], o["gates"], o["route_row"], 2, activation=None)

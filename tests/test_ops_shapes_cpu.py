@@ -26,3 +26,20 @@ def test_router_weight_of_another_width(route, w):
 def test_logits_of_another_shape(logits):
     with pytest.raises(RuntimeError, match="logits must be"):
         ops.fused_select(logits, _half(4, 64), 8, 2)
+
+
+def _int32(*shape):
+    return torch.zeros(*shape, dtype=torch.int32)
+
+
+def test_offsets_of_fewer_experts():
+    with pytest.raises(RuntimeError, match="offsets must have"):
+        ops.grouped_gemm(_half(6, 16), _half(4, 32, 16), _int32(4))
+    with pytest.raises(RuntimeError, match="offsets must have"):
+        ops.expert_ffn(_half(6, 16), _half(4, 32, 16), _half(4, 16, 32), _int32(4), torch.zeros(3, 2), _int32(6), 2, activation=None)
+
+
+@pytest.mark.parametrize("gates,route_row", [((2, 2), 6), ((3, 1), 6), ((3, 3), 6), ((5,), 6), ((3, 2), 5)])
+def test_maps_of_another_routing(gates, route_row):
+    with pytest.raises(RuntimeError, match="combine: "):
+        ops.combine(_half(6, 16), torch.zeros(*gates), _int32(route_row), 2)
