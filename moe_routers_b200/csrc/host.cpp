@@ -387,7 +387,8 @@ PyObject* expert_ffn(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int64_t rows = a->size(0), d = a->size(1), e = w1->size(0);
   const int64_t h = act == MOE_ACT_SWIGLU ? w1->size(1) / 2 : w1->size(1), d2 = w2->size(1);
   const int64_t routes = rows / k * k;
-  if (e == 0 || w1->size(2) != d || w2->size(0) != e || w2->size(2) != h || offsets->numel() <= e || gates->numel() < routes ||
+  // (with an odd number of SwiGLU features an expert's weights are not 2 h rows apart, which moe_expert_ffn assumes)
+  if (e == 0 || (act == MOE_ACT_SWIGLU && w1->size(1) % 2 != 0) || w1->size(2) != d || w2->size(0) != e || w2->size(2) != h || offsets->numel() <= e || gates->numel() < routes ||
       gates->size(1) != k || route_row->numel() < routes) Py_RETURN_NONE;
   c.workspace(args[0], 1, (int)e, 1);
   const int type = type_code(*a);

@@ -67,6 +67,19 @@ def test_expert_ffn(act, t, k):
 
 
 @pytest.mark.gpu
+def test_expert_ffn_with_an_odd_number_of_swiglu_features():
+    """Gate and up rows are the first 2 h of an expert's 2 h + 1; the last one is not used."""
+    from moe_routers_b200 import ops
+
+    e, d, h, k = 4, 128, 64, 2
+    o = ops.route_fused(_randn(24, d), _randn(e, d, seed=1), k)
+    w1, w2 = _randn(e, 2 * h + 1, d, seed=2) / 8, _randn(e, d, h, seed=3) / 8
+    args = o["offsets"], o["gates"], o["route_row"], k
+    _same(ops.expert_ffn(o["packed"], w1, w2, *args, activation="swiglu"),
+          ops.expert_ffn(o["packed"], w1[:, :2 * h].contiguous(), w2, *args, activation="swiglu"))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("counts", [[5], [0, 3, 0, 70, 1], [1] * 100, [2, 0] * 300])
 def test_grouped_lists(counts):
     from moe_routers_b200 import grouped_ffn_cuda, ops
