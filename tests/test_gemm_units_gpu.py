@@ -38,7 +38,11 @@ def test_column_groups(cnt, act):
 
 @pytest.mark.parametrize("experts,rows,n", [
     (1, 128, 256),       # one unit: two pieces
-    (1, 127, 256),       # .. of 64 and 63 tokens
+    (1, 127, 256),       # (with fewer than 128 rows there is one cluster per unit: whole)
+    (1, 250, 5120),      # 20 units: three pieces each
+    (1, 190, 6144),      # 24 units of 192 columns: three pieces each
+    (1, 128, 4864),      # 19 units: three would fit, 128 columns give two
+    (1, 250, 24064),     # 94 units: one full round and 20 in three pieces
     (1, 256, 4608),      # 18 units: four pieces each
     (1, 225, 4608),      # 18 units of 256 columns
     (1, 250, 9472),      # 37 units: two pieces
