@@ -526,6 +526,14 @@ extern "C" int moe_pack_static(const void* x, int elem_bytes, const int32_t* idx
 }
 
 namespace moe {
+namespace {
+bool is_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // (the legacy stream while another thread captures: the launch that follows reports it)
+  return true;
+}
+}  // namespace
 int launch_select_any(const void* logits, int logits_dtype, int tokens, int experts, int top_k, int32_t* idx,
                       float* gates, int32_t* tile_hist, cudaStream_t s, bool early);
 }
@@ -550,11 +558,13 @@ extern "C" int moe_fused_select(const void* logits, int logits_dtype, const void
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Workspace ws = carve(workspace, tokens, experts);
   if (tokens > 0) {
-    // The select sets itself up under the kernel in front (in a sequence of calls: the last scatter) where the rows take
-    // longer than the host's 15 us for a call: calls of 4096 x 4096: 23.1 -> 22.3 us, 8192 x 2048: 24.7 -> 23.5 (in a graph 22.2
-    // and 23.3 -> 23.6).  Smaller calls took the host longer (1024 x 4096: 15.2 -> 18), and with the scan in between
-    // 12000 x 4096 took 56.2 instead of 53.9 us.
-    const bool early = (1LL + top_k) * tokens * d * elem_bytes >= kEarlySelectBytes && ws.num_tiles <= kFusedPrefixTiles;
+    // The select sets itself up under the kernel in front (in a sequence of calls: the last scatter).  Off -> on, us a call, one
+    // call behind the other in a stream: 2731 x 4096: 20.6 -> 17.4, 4096 x 4096: 22.6 -> 20.7, 8192 x 2048: 22.7 -> 22.0.  Smaller
+    // calls are as long as the host takes for them, 13 us, or little longer (1024 x 4096: 13.4 -> 13.0, 2048 x 4096: 14.7 -> 13.1);
+    // behind a scan it loses (12000 x 4096: 55.6 -> 55.9, 16387 x 4096: 72.3 -> 72.8).  In a graph there is hardly a gap between
+    // the kernels to hide it in, and it takes room from the scatter in front: 2731 x 4096: 18.0 -> 18.3, 4096 x 4096: 19.9 ->
+    // 20.3, 8192 x 2048: 20.9 -> 21.7, 8192 x 4096: 39.4 -> 40.6.
+    const bool early = (1LL + top_k) * tokens * d * elem_bytes >= kEarlySelectBytes && ws.num_tiles <= kFusedPrefixTiles && !is_capturing(s);
     const int rc = launch_select_any(logits, logits_dtype, tokens, experts, top_k, idx, gates, ws.tile_hist, s, early);
     if (rc != MOE_OK) return rc;
   }

@@ -1,5 +1,7 @@
 """Kernels that set themselves up, or begin to copy, under the kernel in front of them: the same bits as one kernel after
 another, at sizes where what starts early has to wait in the middle of its work."""
+import ctypes
+
 import pytest
 import torch
 
@@ -103,3 +105,23 @@ def test_layers_behind_one_another(tokens, d, h, e, k):
         for a, b in zip(chain(x), want):
             _same(a, b)
     assert ops.read_status() == 0
+
+
+def test_a_captured_select_is_launched_plainly():
+    """Among the kernels of a graph an early start of the select costs time: only the scatters start under their selects."""
+    from moe_routers_b200 import ops
+
+    x, logits = _randn(4096, 4096), _randn(4096, 64, seed=1)
+    want = ops.fused_select(logits, x, 64, 2)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        got = [ops.fused_select(logits, x, 64, 2) for _ in range(3)]
+    driver, count = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t(16)
+    nodes, edges = [(ctypes.c_void_p * 16)() for _ in range(2)], (ctypes.c_ubyte * 8 * 16)()  # from_port, to_port, type, ..
+    assert driver.cuGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), *nodes, edges, ctypes.byref(count)) == 0
+    assert [e[2] for e in edges[:count.value]].count(1) == 3  # 1: CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC
+    graph.instantiate()
+    graph.replay()
+    for outs in got:
+        for a, b in zip(outs, want):
+            _same(a, b)
