@@ -461,9 +461,12 @@ def combine_dense(y: torch.Tensor, idx: torch.Tensor, gates: torch.Tensor, exper
     dev = y.get_device()
     with _on(dev):
         out, = empties(dev, ((y.dtype, t, d),))
+        stream = _stream()
+        ws = _workspaces.get((dev, stream))  # (of any size: only its status word is used)
+        if ws is None:
+            ws = _workspace(dev, 1, 1, 1)
         check(lib.moe_combine_dense_checked(y.data_ptr(), _DTYPE_CODE[y.dtype], idx.data_ptr(), gates.data_ptr(), t, d,
-                                            int(experts), idx.size(1), out.data_ptr(), _workspace(dev, 1, 1, 1).data_ptr(),
-                                            _stream()))
+                                            int(experts), idx.size(1), out.data_ptr(), ws.data_ptr(), stream))
     return out
 
 

@@ -50,15 +50,18 @@ def masked_matmul_forward(x: torch.Tensor, r: dict, w1: torch.Tensor, w2: torch.
     e = w1.size(0)
     if e > 8:
         raise RuntimeError("masked_matmul_forward supports at most 8 experts")
-    y = torch.empty((e * t, d), dtype=x.dtype, device=x.device)
     # All experts in one pair of launches, or as many at a time as keep the hidden rows within the bound.  One pair per
     # expert filled its last round of units each time, and the mask took four launches: 8 experts x 281 tokens,
     # 1792 -> 1152: 283 -> 59 us; 4 x 1389, 2368 -> 7264: 455 -> 388; 8 x 4096, 4096 -> 8192: 3865 -> 3755.
     at_once = max(1, _HIDDEN_BYTES // max(1, t * w1.size(1) * x.element_size()))
-    for e0 in range(0, e, at_once):
-        e1 = min(e, e0 + at_once)
-        h = ops.dense_experts(x, w1[e0:e1], t, activation=activation)
-        ops.dense_experts(h, w2[e0:e1], t, out=y[e0 * t:e1 * t])
+    if at_once >= e:  # (without slices, which take the host longer than the checks of what they give)
+        y = ops.dense_experts(ops.dense_experts(x, w1, t, activation=activation), w2, t)
+    else:
+        y = torch.empty((e * t, d), dtype=x.dtype, device=x.device)
+        for e0 in range(0, e, at_once):
+            e1 = min(e, e0 + at_once)
+            h = ops.dense_experts(x, w1[e0:e1], t, activation=activation)
+            ops.dense_experts(h, w2[e0:e1], t, out=y[e0 * t:e1 * t])
     idx, gates = r["idx"], r["gates"]
     if not (idx.dim() == 2 and idx.shape == gates.shape and idx.size(0) == t and 1 <= idx.size(1) <= 8
             and idx.device == gates.device == x.device):
