@@ -55,9 +55,6 @@ combine_vec_kernel(const uint4* __restrict__ y, const float* __restrict__ gates,
   const int v_begin = SPLIT ? blockIdx.y * part_vec : 0;  // this warp's 16-byte pieces of the row
   const int n_vec = SPLIT ? min(n_vec_total, v_begin + part_vec) : n_vec_total;
   const int top_k = TOPK > 0 ? TOPK : top_k_rt;
-  if constexpr (DENSE) {
-    if (lane < picks && (unsigned)__ldg(route_row + (size_t)t * picks + lane) >= (unsigned)top_k) record_error(status, kErrBadIndex);
-  }
   const uint4* src[8];
   float g[8];
 #pragma unroll
@@ -117,6 +114,9 @@ combine_vec_kernel(const uint4* __restrict__ y, const float* __restrict__ gates,
         dst[v0 + u * 32] = o;
       }
     }
+  }
+  if constexpr (DENSE) {  // (at the end, where nothing waits for it)
+    if (lane < picks && (unsigned)__ldg(route_row + (size_t)t * picks + lane) >= (unsigned)top_k) record_error(status, kErrBadIndex);
   }
 }
 
